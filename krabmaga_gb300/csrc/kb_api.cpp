@@ -442,6 +442,14 @@ kb_status reset_wait_state(kb_field* f) {
     return KB_OK;
 }
 
+// The arrival slots a force pass keeps for the ranked rebin; nullptr for dense
+// flocks, which rebin by segments: most of their boids share a bag with more
+// than RANK_SLOTS others, and each of those would walk its source lines (at
+// the 48-candidate switch a mean bag holds five).
+uint32_t* rank_slots(const kb_field* f) {
+    return f->dense && f->reps.size() == 1 ? nullptr : f->slots.p;
+}
+
 // The general stable sort: write list -> read buffer.  hist already holds
 // the key counts when counted == true.
 kb_status general_rebuild(kb_field* f, bool counted) {
@@ -487,6 +495,7 @@ kb_status fast_rebuild(kb_field* f, bool bump_step) {
     a.step = bump_step ? f->dstep.p : nullptr;
     a.err = f->err.p;
     a.n = f->rn;
+    a.slots = f->slots_kept ? f->slots.p : nullptr;
     KB_CUDA(launch_rebin(a, s));
     f->cur = nxt;
     return KB_OK;
@@ -506,6 +515,9 @@ kb_status enqueue_force(kb_field* f, const kb_flock_params* p) {
     a.out_ids = f->wid.p;
     a.out_key = f->wkey.p;
     a.hist = f->hist.p;
+    a.slots = rank_slots(f);
+    a.ncells = f->ncells_total;
+    f->slots_kept = a.slots != nullptr;
     a.err = f->err.p;
     // The fast rebin is used only when |jump| * 1.001 < d, so no boid can
     // leave the 3x3 stencil; the rebin's own count check (every bag gathers
@@ -975,6 +987,7 @@ kb_status field_new(int device, const std::vector<Rep>& reps, bool is_batch, uin
     if (!e) e = f->start[1].alloc((size_t)nc + 1);
     if (!e) e = f->hist.alloc(nc);
     if (!e) e = f->cursor.alloc(nc);
+    if (!e && nc <= RANK_MAX_CELLS) e = f->slots.alloc((size_t)nc * RANK_SLOTS);
     if (!e) e = f->scan_ctl.alloc(1);
     if (!e) e = f->aux_ctl.alloc(1);
     if (!e) e = f->tstate.alloc(nt);
@@ -1018,11 +1031,12 @@ kb_status grow_cells(kb_field* f, uint64_t need) {
     if (need > 0xF0000000ull) return fail(KB_ERR_ARG, "bag matrix too large");
     const uint32_t nc = (uint32_t)std::min<uint64_t>(0xF0000000ull, std::max<uint64_t>(need, 2ull * f->cells_cap));
     const uint32_t nt = scan_state_words(nc);
-    DevBuf<uint32_t> s0, s1, hist, cursor;
+    DevBuf<uint32_t> s0, s1, hist, cursor, slots;
     DevBuf<unsigned long long> ts;
     cudaError_t e;
     if ((e = s0.alloc((size_t)nc + 1)) || (e = s1.alloc((size_t)nc + 1)) || (e = hist.alloc(nc)) ||
-        (e = cursor.alloc(nc)) || (e = ts.alloc(nt)))
+        (e = cursor.alloc(nc)) || (e = ts.alloc(nt)) ||
+        (nc <= RANK_MAX_CELLS && (e = slots.alloc((size_t)nc * RANK_SLOTS))))
         return cuda_fail(e, "growing the bag arrays");
     KB_CUDA(cudaMemsetAsync(s0.p, 0, sizeof(uint32_t) * ((size_t)nc + 1), f->stream));
     KB_CUDA(cudaMemsetAsync(s1.p, 0, sizeof(uint32_t) * ((size_t)nc + 1), f->stream));
@@ -1034,6 +1048,7 @@ kb_status grow_cells(kb_field* f, uint64_t need) {
     f->start[1].swap(s1);
     f->hist.swap(hist);
     f->cursor.swap(cursor);
+    f->slots.swap(slots);
     f->tstate.swap(ts);
     f->cells_cap = nc;
     f->hist_counted = false;

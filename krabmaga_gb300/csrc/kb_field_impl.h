@@ -51,6 +51,10 @@ struct kb_field {
     bool p_loc_differs = false;
     // step temporaries
     DevBuf<uint32_t> hist, cursor, tid, tsrc, rkey, tkey;
+    // arrival slots of the ranked rebin, RANK_SLOTS per bag (empty above
+    // RANK_MAX_CELLS bags: those fields rebin by segments)
+    DevBuf<uint32_t> slots;
+    bool slots_kept = false;  // the last force pass left its arrivals in slots
     bool hist_counted = false;  // a force pass has counted arrivals into hist (no scan since)
     // Every replica's ids are distinct in the read buffer (checked on the
     // device after each general rebuild; the step paths keep the id multiset)

@@ -191,7 +191,7 @@ __device__ __noinline__ void columns_runs_5(const ForceArgs& a, const Rep& R, in
     columns_runs<5>(a, R, mi, Mi, mj, Mj, me, my_id, acc);
 }
 
-template <bool STRICT>
+template <bool STRICT, bool SLOTS>
 __device__ __forceinline__ void force_finish(const ForceArgs& a, const Rep& R, uint32_t i,
                                              float4 me, uint32_t my_id, unsigned long long step,
                                              const Acc<STRICT>& acc);
@@ -260,12 +260,13 @@ __device__ __forceinline__ void force_body(const ForceArgs& a, const Rep& R, uin
     const uint32_t my_id = __ldg(a.ids + i);
     Acc<STRICT> acc;
     gather_candidates<STRICT, QMODE, DENSE>(a, R, me, my_id, a.self_by_slot ? i : 0xFFFFFFFFu, acc);
-    force_finish<STRICT>(a, R, i, me, my_id, step, acc);
+    force_finish<STRICT, !DENSE>(a, R, i, me, my_id, step, acc);
 }
 
 // bird.rs:84-153 after the candidate sums: the next state at slot i of the
-// write list, its bag key and the arrival count of that bag.
-template <bool STRICT>
+// write list, its bag key and the arrival count of that bag.  SLOTS: a's
+// arrival slots are kept where it has them.
+template <bool STRICT, bool SLOTS>
 __device__ __forceinline__ void force_finish(const ForceArgs& a, const Rep& R, uint32_t i,
                                              float4 me, uint32_t my_id, unsigned long long step,
                                              const Acc<STRICT>& acc) {
@@ -291,7 +292,13 @@ __device__ __forceinline__ void force_finish(const ForceArgs& a, const Rep& R, u
     if (flags) atomicOr(a.err, flags);
     const uint32_t key = R.cell_off + (uint32_t)idx;
     a.out_key[i] = key;
-    atomicAdd(&a.hist[key], 1u);
+    if (SLOTS && a.slots) {
+        const uint32_t r = atomicAdd(&a.hist[key], 1u);
+        if (r < RANK_ROW) a.slots[(size_t)key * RANK_ROW + r] = i;
+        else if (r < RANK_SLOTS) a.slots[(size_t)a.ncells * RANK_ROW + (size_t)key * RANK_ROW2 + (r - RANK_ROW)] = i;
+    } else {
+        atomicAdd(&a.hist[key], 1u);
+    }
 }
 
 #ifndef KB_FORCE_THREADS
@@ -350,7 +357,7 @@ __global__ void __launch_bounds__(KB_FORCE_THREADS)
     const uint32_t my_id = in_ids[j];
     Acc<STRICT> acc;
     gather_candidates<STRICT, QMODE>(a, a.rep0, me, my_id, 0xFFFFFFFFu, acc);
-    force_finish<STRICT>(a, a.rep0, j, me, my_id, step, acc);
+    force_finish<STRICT, false>(a, a.rep0, j, me, my_id, step, acc);
 }
 
 // Mark every live write-list entry whose id is in sorted[0..m) removed.
@@ -1084,6 +1091,101 @@ __global__ void __launch_bounds__(32 * REBIN_SEG_WARPS, MULTI ? KB_REBIN_MINB_MU
     rebin_segment<ROWS>(a, a.rep0, g, s_cnt[w]);
 }
 
+// ---------------------------------------------------------- ranked rebin
+// One thread per write-list entry: its place in its next bag is the bag's
+// next offset plus the number of arrivals of that bag that come before it in
+// the list (the insertion order of the reference's lazy_update).  The force
+// pass left the first RANK_SLOTS arrivals of every bag in a.slots, in no
+// particular order, so a bag of at most RANK_ROW needs one 16-byte load and
+// four compares, one of at most RANK_SLOTS two loads more.  A fuller bag
+// counts its arrivals in the source lines of src_line, as the segment rebin
+// does.  Bound by load latency and, at 1M boids, by the L2's capacity: the
+// segment rebin's dependent rounds (offsets, keys, ranks, records) become two
+// (key and record; offsets and slots).  Measured per step, force and scan
+// included (us, segments against ranks): 20k boids 13.2 / 8.9, 262k 24.2 /
+// 17.0, 1M 53.3 / 44.3, 1M at density 0.06 59.6 / 52.8; 512 packed replicas
+// (8.4M boids) 592 / 511.  The force pass pays 1.5 of the 1M step's us for
+// the slots (its counting atomics return a value).
+__device__ __noinline__ uint32_t rank_by_lines(const RebinArgs& a, const Rep& R, uint32_t key,
+                                               uint32_t i, uint32_t cnt) {
+    const uint32_t local = key - R.cell_off;
+    const uint32_t Xu = div_dh(local, R);
+    const int X = (int)Xu, Y = (int)(local - Xu * (uint32_t)R.dh);
+    uint32_t rank = 0, total = 0;
+    auto count = [&](uint32_t s, uint32_t e) {
+        for (uint32_t p = s; p < e; ++p) {
+            const uint32_t m = __ldg(a.key + p) == key ? 1u : 0u;
+            total += m;
+            rank += p < i ? m : 0u;
+        }
+    };
+    if (X > 0 && X < R.seam && Y > 0 && Y < R.seam) {
+#pragma unroll 1
+        for (int k = -1; k <= 1; ++k) {
+            const uint32_t c = R.cell_off + (uint32_t)(X + k) * (uint32_t)R.dh + (uint32_t)Y;
+            const uint32_t e = min(__ldg(a.start_cur + c + 2), a.n);
+            count(min(__ldg(a.start_cur + c - 1), e), e);
+        }
+    } else {
+        int lastx = -1;
+#pragma unroll 1
+        for (int kx = 0; kx < SRC_LINES; ++kx) {
+            const int sx = src_line(kx, X, R.max_x, R.seam);
+            if (sx < 0 || sx > R.max_x || sx <= lastx) continue;
+            lastx = sx;
+            const uint32_t colbase = R.cell_off + (uint32_t)sx * (uint32_t)R.dh;
+            int lasty = -1;
+#pragma unroll 1
+            for (int ky = 0; ky < SRC_LINES; ++ky) {
+                const int sy = src_line(ky, Y, R.max_y, R.seam);
+                if (sy < 0 || sy > R.max_y || sy <= lasty) continue;
+                lasty = sy;
+                const uint32_t e = min(__ldg(a.start_cur + colbase + sy + 1), a.n);
+                count(min(__ldg(a.start_cur + colbase + sy), e), e);
+            }
+        }
+    }
+    if (total != cnt) atomicOr(a.err, ERR_REBIN_MISS | ERR_MISS_MATERIALIZE);
+    return rank;
+}
+
+template <bool MULTI>
+__global__ void __launch_bounds__(256) k_rebin_rank(RebinArgs a) {
+    static_assert(RANK_ROW == 4 && RANK_ROW2 == 8, "the rows are read 16 bytes at a time");
+    pdl_enter();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0 && a.step != nullptr) *a.step += 1ull;
+    if (i >= a.n) return;
+    const uint32_t key = __ldg(a.key + i);
+    const float4 rec = __ldg(a.a_st + i);
+    const uint32_t id = __ldg(a.a_ids + i);
+    const uint32_t e = min(__ldg(a.start_next + key + 1), a.n);
+    const uint32_t s = min(__ldg(a.start_next + key), e);
+    const uint32_t cnt = e - s;
+    uint32_t rank = 0;
+    if (cnt > RANK_SLOTS) {
+        if (MULTI) rank = rank_by_lines(a, a.reps[rep_of_cell(a.reps, a.nrep, key)], key, i, cnt);
+        else rank = rank_by_lines(a, a.rep0, key, i, cnt);
+    } else if (cnt > 1u) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(a.slots) + key);
+        rank = (v.x < i) + (v.y < i) + (cnt > 2u && v.z < i) + (cnt > 3u && v.w < i);
+        if (cnt > RANK_ROW) {
+            const uint4* row = reinterpret_cast<const uint4*>(a.slots) + (size_t)a.ncells + 2u * (size_t)key;
+            const uint4 u = __ldg(row);
+            rank += (u.x < i) + (cnt > 5u && u.y < i) + (cnt > 6u && u.z < i) + (cnt > 7u && u.w < i);
+            if (cnt > 8u) {
+                const uint4 t = __ldg(row + 1);
+                rank += (t.x < i) + (cnt > 9u && t.y < i) + (cnt > 10u && t.z < i) + (cnt > 11u && t.w < i);
+            }
+        }
+    }
+    const uint32_t dst = s + rank;
+    if (dst < a.n) {
+        a.s_st[dst] = rec;
+        a.s_ids[dst] = id;
+    }
+}
+
 // Sum of squared bag occupancies of a read buffer (its offsets), a measure
 // of how long the candidate lists are: about 9 * sum / N per boid.
 __global__ void k_occupancy_sq(const uint32_t* __restrict__ start, uint32_t ncells,
@@ -1591,6 +1693,12 @@ cudaError_t launch_remove_ids(const uint32_t* ids, uint8_t* dead, uint32_t n, co
 }
 
 cudaError_t launch_rebin(const RebinArgs& a, cudaStream_t s) {
+    if (a.slots != nullptr) {
+        if (a.key == nullptr && a.n > 0) return cudaErrorInvalidValue;
+        const unsigned gr = grid_for(a.n > 0 ? a.n : 1, 256);
+        return a.nrep > 1 ? launch_pdl(k_rebin_rank<true>, gr, 256, s, a)
+                          : launch_pdl(k_rebin_rank<false>, gr, 256, s, a);
+    }
     if (a.key != nullptr && a.nsegs > 0 && (a.nrep == 1 || a.sblk != nullptr)) {
         if (a.nrep > 1) return launch_pdl(k_rebin_seg<true>, a.nsblk, 32 * REBIN_SEG_WARPS, s, a);
         const unsigned gs = grid_for(a.nsegs, REBIN_SEG_WARPS);

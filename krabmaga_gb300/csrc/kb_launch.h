@@ -74,6 +74,10 @@ struct ForceArgs {
     uint32_t* out_ids;
     uint32_t* out_key;
     uint32_t* hist;
+    // the first RANK_SLOTS arrivals of every bag (their write-list slots, in
+    // the order the counts were taken), for the ranked rebin; nullptr: not kept
+    uint32_t* slots;
+    uint32_t ncells;  // bags over all replicas (the second row of a.slots starts behind them)
     uint32_t* err;
     int32_t check_moves;  // flag moves the stencil-gather rebin cannot follow
     // several replicas: one block per entry {replica, first boid}; no block
@@ -152,7 +156,17 @@ struct RebinArgs {
     unsigned long long* step;
     uint32_t* err;
     uint32_t n;  // records (every slot index is below it)
+    const uint32_t* slots;  // the force pass's arrival slots: the ranked rebin (nullptr: by segments)
 };
+// Arrivals per bag whose write-list slots the force pass records: the first
+// four of every bag in one array of 16 B per bag, the next eight in a second
+// one of 32 B per bag behind it that bags of ordinary occupancy never touch.
+// (A single row of 8 or 16 per bag ran the 1M step at 47.2 or 52.0 us against
+// 44.6 us for a row of 4: the step's working set is near the L2's size.)
+constexpr uint32_t RANK_ROW = 4, RANK_ROW2 = 8;
+constexpr uint32_t RANK_SLOTS = RANK_ROW + RANK_ROW2;
+// Bag matrices up to this many bags carry the arrival slots (48 B per bag).
+constexpr uint32_t RANK_MAX_CELLS = 1u << 26;
 // Bag segments of the segment rebin: SEG_ROWS consecutive bags of one column.
 constexpr int SEG_ROWS = 32;
 // Shorter segments for dense flocks: a segment's source runs are long there,
