@@ -1101,7 +1101,8 @@ __global__ void __launch_bounds__(32 * REBIN_SEG_WARPS, MULTI ? KB_REBIN_MINB_MU
 // counts its arrivals in the source lines of src_line, as the segment rebin
 // does.  Bound by load latency and, at 1M boids, by the L2's capacity: the
 // segment rebin's dependent rounds (offsets, keys, ranks, records) become two
-// (key and record; offsets and slots).  Measured per step, force and scan
+// (key and record, read while the scan still runs; offsets and slots).
+// Measured per step, force and scan
 // included (us, segments against ranks): 20k boids 13.2 / 8.9, 262k 24.2 /
 // 17.0, 1M 53.3 / 44.3, 1M at density 0.06 59.6 / 52.8; 512 packed replicas
 // (8.4M boids) 592 / 511.  The force pass pays 1.5 of the 1M step's us for
@@ -1152,13 +1153,20 @@ __device__ __noinline__ uint32_t rank_by_lines(const RebinArgs& a, const Rep& R,
 template <bool MULTI>
 __global__ void __launch_bounds__(256) k_rebin_rank(RebinArgs a) {
     static_assert(RANK_ROW == 4 && RANK_ROW2 == 8, "the rows are read 16 bytes at a time");
-    pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t key = 0, id = 0;
+    float4 rec = {};
+    // the write list is the force pass's: the offsets scan in between has
+    // waited for that pass before it let this kernel start, so the list is
+    // read while the scan still runs
+    if (i < a.n) {
+        key = __ldcg(a.key + i);
+        rec = __ldcg(a.a_st + i);
+        id = __ldcg(a.a_ids + i);
+    }
+    pdl_enter();
     if (i == 0 && a.step != nullptr) *a.step += 1ull;
     if (i >= a.n) return;
-    const uint32_t key = __ldg(a.key + i);
-    const float4 rec = __ldg(a.a_st + i);
-    const uint32_t id = __ldg(a.a_ids + i);
     const uint32_t e = min(__ldg(a.start_next + key + 1), a.n);
     const uint32_t s = min(__ldg(a.start_next + key), e);
     const uint32_t cnt = e - s;
