@@ -444,8 +444,8 @@ kb_status reset_wait_state(kb_field* f) {
 
 // The arrival slots a force pass keeps for the ranked rebin; nullptr for dense
 // flocks, which rebin by segments: most of their boids share a bag with more
-// than RANK_SLOTS others, and each of those would walk its source lines (at
-// the 48-candidate switch a mean bag holds five).
+// than RANK_SLOTS others, and every key of a warp would walk its source lines
+// (4M clustered boids: rebin 238 us by ranks, 160 us by 8-bag segments).
 uint32_t* rank_slots(const kb_field* f) {
     return f->dense && f->reps.size() == 1 ? nullptr : f->slots.p;
 }

@@ -1092,13 +1092,13 @@ __global__ void __launch_bounds__(32 * REBIN_SEG_WARPS, MULTI ? KB_REBIN_MINB_MU
 }
 
 // ---------------------------------------------------------- ranked rebin
-// One thread per write-list entry: its place in its next bag is the bag's
+// Each write-list entry: its place in its next bag is the bag's
 // next offset plus the number of arrivals of that bag that come before it in
 // the list (the insertion order of the reference's lazy_update).  The force
 // pass left the first RANK_SLOTS arrivals of every bag in a.slots, in no
 // particular order, so a bag of at most RANK_ROW needs one 16-byte load and
-// four compares, one of at most RANK_SLOTS two loads more.  A fuller bag
-// counts its arrivals in the source lines of src_line, as the segment rebin
+// four compares, one of at most RANK_SLOTS two loads more.  The arrivals of a
+// fuller bag are counted in the source lines of src_line, as the segment rebin
 // does.  Bound by load latency and, at 1M boids, by the L2's capacity: the
 // segment rebin's dependent rounds (offsets, keys, ranks, records) become two
 // (key and record, read while the scan still runs; offsets and slots).
@@ -1107,91 +1107,147 @@ __global__ void __launch_bounds__(32 * REBIN_SEG_WARPS, MULTI ? KB_REBIN_MINB_MU
 // 17.0, 1M 53.3 / 44.3, 1M at density 0.06 59.6 / 52.8; 512 packed replicas
 // (8.4M boids) 592 / 511.  The force pass pays 1.5 of the 1M step's us for
 // the slots (its counting atomics return a value).
-__device__ __noinline__ uint32_t rank_by_lines(const RebinArgs& a, const Rep& R, uint32_t key,
-                                               uint32_t i, uint32_t cnt) {
-    const uint32_t local = key - R.cell_off;
-    const uint32_t Xu = div_dh(local, R);
-    const int X = (int)Xu, Y = (int)(local - Xu * (uint32_t)R.dh);
-    uint32_t rank = 0, total = 0;
-    auto count = [&](uint32_t s, uint32_t e) {
-        for (uint32_t p = s; p < e; ++p) {
-            const uint32_t m = __ldg(a.key + p) == key ? 1u : 0u;
-            total += m;
-            rank += p < i ? m : 0u;
-        }
-    };
-    if (X > 0 && X < R.seam && Y > 0 && Y < R.seam) {
+//
+// Fuller bags: the warp takes its distinct keys in turn; for each it reads the
+// bag's source lines 32 entries at a time, and every lane of that key counts
+// the arrivals before its own entry.  Every lane of the warp calls it with its
+// entry i (over: the entry's bag is a fuller one).  Out of line and after the
+// others are written, so that it costs them no registers.
+template <bool MULTI>
+__device__ __noinline__ void place_by_lines(const RebinArgs& a, bool over, uint32_t i) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t key = 0, first = 0, cnt = 0, rank = 0;
+    if (over) {
+        key = __ldcg(a.key + i);
+        first = __ldg(a.start_next + key);
+        cnt = min(__ldg(a.start_next + key + 1), a.n) - first;
+    }
+    uint32_t pending = __ballot_sync(FULL_MASK, over);
+    while (pending) {
+        const uint32_t leader = __ffs(pending) - 1;
+        const uint32_t k = __shfl_sync(FULL_MASK, key, leader);
+        const bool mine = over && key == k;
+        const Rep& R = MULTI ? a.reps[rep_of_cell(a.reps, a.nrep, k)] : a.rep0;
+        const uint32_t local = k - R.cell_off;
+        const uint32_t Xu = div_dh(local, R);
+        const int X = (int)Xu, Y = (int)(local - Xu * (uint32_t)R.dh);
+        uint32_t total = 0;
+        auto count = [&](uint32_t s, uint32_t e) {
+#pragma unroll 2
+            for (uint32_t p = s; p < e; p += 32u) {
+                const bool hit = p + lane < e && __ldg(a.key + p + lane) == k;
+                const uint32_t m = __ballot_sync(FULL_MASK, hit);
+                total += __popc(m);
+                // entries p .. i-1 of this batch
+                const uint32_t d = i > p ? i - p : 0u;
+                rank += mine ? __popc(d >= 32u ? m : m & ((1u << d) - 1u)) : 0;
+            }
+        };
+        if (X > 0 && X < R.seam && Y > 0 && Y < R.seam) {
 #pragma unroll 1
-        for (int k = -1; k <= 1; ++k) {
-            const uint32_t c = R.cell_off + (uint32_t)(X + k) * (uint32_t)R.dh + (uint32_t)Y;
-            const uint32_t e = min(__ldg(a.start_cur + c + 2), a.n);
-            count(min(__ldg(a.start_cur + c - 1), e), e);
-        }
-    } else {
-        int lastx = -1;
+            for (int q = -1; q <= 1; ++q) {
+                const uint32_t c = R.cell_off + (uint32_t)(X + q) * (uint32_t)R.dh + (uint32_t)Y;
+                const uint32_t e = min(__ldg(a.start_cur + c + 2), a.n);
+                count(min(__ldg(a.start_cur + c - 1), e), e);
+            }
+        } else {
+            int lastx = -1;
 #pragma unroll 1
-        for (int kx = 0; kx < SRC_LINES; ++kx) {
-            const int sx = src_line(kx, X, R.max_x, R.seam);
-            if (sx < 0 || sx > R.max_x || sx <= lastx) continue;
-            lastx = sx;
-            const uint32_t colbase = R.cell_off + (uint32_t)sx * (uint32_t)R.dh;
-            int lasty = -1;
+            for (int kx = 0; kx < SRC_LINES; ++kx) {
+                const int sx = src_line(kx, X, R.max_x, R.seam);
+                if (sx < 0 || sx > R.max_x || sx <= lastx) continue;
+                lastx = sx;
+                const uint32_t colbase = R.cell_off + (uint32_t)sx * (uint32_t)R.dh;
+                int lasty = -1;
 #pragma unroll 1
-            for (int ky = 0; ky < SRC_LINES; ++ky) {
-                const int sy = src_line(ky, Y, R.max_y, R.seam);
-                if (sy < 0 || sy > R.max_y || sy <= lasty) continue;
-                lasty = sy;
-                const uint32_t e = min(__ldg(a.start_cur + colbase + sy + 1), a.n);
-                count(min(__ldg(a.start_cur + colbase + sy), e), e);
+                for (int ky = 0; ky < SRC_LINES; ++ky) {
+                    const int sy = src_line(ky, Y, R.max_y, R.seam);
+                    if (sy < 0 || sy > R.max_y || sy <= lasty) continue;
+                    lasty = sy;
+                    const uint32_t e = min(__ldg(a.start_cur + colbase + sy + 1), a.n);
+                    count(min(__ldg(a.start_cur + colbase + sy), e), e);
+                }
             }
         }
+        if (mine && total != cnt) atomicOr(a.err, ERR_REBIN_MISS | ERR_MISS_MATERIALIZE);
+        pending &= ~__ballot_sync(FULL_MASK, mine);
     }
-    if (total != cnt) atomicOr(a.err, ERR_REBIN_MISS | ERR_MISS_MATERIALIZE);
-    return rank;
+    if (over && first + rank < a.n) {
+        a.s_st[first + rank] = __ldcg(a.a_st + i);
+        a.s_ids[first + rank] = __ldcg(a.a_ids + i);
+    }
 }
 
+// Two entries per thread, their loads in flight together: a block of 256
+// entries is over in about the time it takes to launch (1M boids: rebin 15.1 us
+// with one entry per thread, 13.0 with two, 15.3 with four; step 43.8 / 41.9 /
+// 43.6 us).  Fuller bags by warps rather than by each boid alone: 64 replicas
+// whose flocks condense over 500 steps, last 100 steps 105 us each against 113
+// for 64-bag segments (per-boid walks: no gain over segments there).
+constexpr int RANK_ITEMS = 2;
+constexpr int RANK_THREADS = 256;
 template <bool MULTI>
-__global__ void __launch_bounds__(256) k_rebin_rank(RebinArgs a) {
+__global__ void __launch_bounds__(RANK_THREADS) k_rebin_rank(RebinArgs a) {
     static_assert(RANK_ROW == 4 && RANK_ROW2 == 8, "the rows are read 16 bytes at a time");
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t key = 0, id = 0;
-    float4 rec = {};
+    const uint32_t i0 = blockIdx.x * (RANK_THREADS * RANK_ITEMS) + threadIdx.x;
+    uint32_t key[RANK_ITEMS], id[RANK_ITEMS];
+    float4 rec[RANK_ITEMS];
     // the write list is the force pass's: the offsets scan in between has
     // waited for that pass before it let this kernel start, so the list is
     // read while the scan still runs
-    if (i < a.n) {
-        key = __ldcg(a.key + i);
-        rec = __ldcg(a.a_st + i);
-        id = __ldcg(a.a_ids + i);
-    }
-    pdl_enter();
-    if (i == 0 && a.step != nullptr) *a.step += 1ull;
-    if (i >= a.n) return;
-    const uint32_t e = min(__ldg(a.start_next + key + 1), a.n);
-    const uint32_t s = min(__ldg(a.start_next + key), e);
-    const uint32_t cnt = e - s;
-    uint32_t rank = 0;
-    if (cnt > RANK_SLOTS) {
-        if (MULTI) rank = rank_by_lines(a, a.reps[rep_of_cell(a.reps, a.nrep, key)], key, i, cnt);
-        else rank = rank_by_lines(a, a.rep0, key, i, cnt);
-    } else if (cnt > 1u) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(a.slots) + key);
-        rank = (v.x < i) + (v.y < i) + (cnt > 2u && v.z < i) + (cnt > 3u && v.w < i);
-        if (cnt > RANK_ROW) {
-            const uint4* row = reinterpret_cast<const uint4*>(a.slots) + (size_t)a.ncells + 2u * (size_t)key;
-            const uint4 u = __ldg(row);
-            rank += (u.x < i) + (cnt > 5u && u.y < i) + (cnt > 6u && u.z < i) + (cnt > 7u && u.w < i);
-            if (cnt > 8u) {
-                const uint4 t = __ldg(row + 1);
-                rank += (t.x < i) + (cnt > 9u && t.y < i) + (cnt > 10u && t.z < i) + (cnt > 11u && t.w < i);
-            }
+#pragma unroll
+    for (int t = 0; t < RANK_ITEMS; ++t) {
+        const uint32_t i = i0 + t * RANK_THREADS;
+        if (i < a.n) {
+            key[t] = __ldcg(a.key + i);
+            rec[t] = __ldcg(a.a_st + i);
+            id[t] = __ldcg(a.a_ids + i);
         }
     }
-    const uint32_t dst = s + rank;
-    if (dst < a.n) {
-        a.s_st[dst] = rec;
-        a.s_ids[dst] = id;
+    pdl_enter();
+    if (i0 == 0 && a.step != nullptr) *a.step += 1ull;
+    uint32_t s[RANK_ITEMS], cnt[RANK_ITEMS];
+#pragma unroll
+    for (int t = 0; t < RANK_ITEMS; ++t) {
+        s[t] = cnt[t] = 0u;
+        if (i0 + t * RANK_THREADS < a.n) {
+            const uint32_t e = min(__ldg(a.start_next + key[t] + 1), a.n);
+            s[t] = min(__ldg(a.start_next + key[t]), e);
+            cnt[t] = e - s[t];
+        }
     }
+    uint4 row[RANK_ITEMS];
+#pragma unroll
+    for (int t = 0; t < RANK_ITEMS; ++t)
+        if (cnt[t] > 1u) row[t] = __ldg(reinterpret_cast<const uint4*>(a.slots) + key[t]);
+#pragma unroll
+    for (int t = 0; t < RANK_ITEMS; ++t) {
+        const uint32_t i = i0 + t * RANK_THREADS, c = cnt[t];
+        if (c > RANK_SLOTS) continue;
+        uint32_t rank = 0;
+        if (c > 1u) {
+            const uint4 v = row[t];
+            rank = (v.x < i) + (v.y < i) + (c > 2u && v.z < i) + (c > 3u && v.w < i);
+            if (c > RANK_ROW) {
+                const uint4* row2 = reinterpret_cast<const uint4*>(a.slots) + (size_t)a.ncells + 2u * (size_t)key[t];
+                const uint4 u = __ldg(row2);
+                rank += (u.x < i) + (c > 5u && u.y < i) + (c > 6u && u.z < i) + (c > 7u && u.w < i);
+                if (c > 8u) {
+                    const uint4 w = __ldg(row2 + 1);
+                    rank += (w.x < i) + (c > 9u && w.y < i) + (c > 10u && w.z < i) + (c > 11u && w.w < i);
+                }
+            }
+        }
+        const uint32_t dst = s[t] + rank;
+        if (i < a.n && dst < a.n) {
+            a.s_st[dst] = rec[t];
+            a.s_ids[dst] = id[t];
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < RANK_ITEMS; ++t)
+        if (__any_sync(FULL_MASK, cnt[t] > RANK_SLOTS))
+            place_by_lines<MULTI>(a, cnt[t] > RANK_SLOTS, i0 + t * RANK_THREADS);
 }
 
 // Sum of squared bag occupancies of a read buffer (its offsets), a measure
@@ -1703,9 +1759,9 @@ cudaError_t launch_remove_ids(const uint32_t* ids, uint8_t* dead, uint32_t n, co
 cudaError_t launch_rebin(const RebinArgs& a, cudaStream_t s) {
     if (a.slots != nullptr) {
         if (a.key == nullptr && a.n > 0) return cudaErrorInvalidValue;
-        const unsigned gr = grid_for(a.n > 0 ? a.n : 1, 256);
-        return a.nrep > 1 ? launch_pdl(k_rebin_rank<true>, gr, 256, s, a)
-                          : launch_pdl(k_rebin_rank<false>, gr, 256, s, a);
+        const unsigned gr = grid_for(a.n > 0 ? a.n : 1, RANK_THREADS * RANK_ITEMS);
+        return a.nrep > 1 ? launch_pdl(k_rebin_rank<true>, gr, RANK_THREADS, s, a)
+                          : launch_pdl(k_rebin_rank<false>, gr, RANK_THREADS, s, a);
     }
     if (a.key != nullptr && a.nsegs > 0 && (a.nrep == 1 || a.sblk != nullptr)) {
         if (a.nrep > 1) return launch_pdl(k_rebin_seg<true>, a.nsblk, 32 * REBIN_SEG_WARPS, s, a);
