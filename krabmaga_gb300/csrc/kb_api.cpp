@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <limits>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -101,6 +102,19 @@ bool make_rep_geometry(float w, float h, float d, int toroidal, Rep* R, std::str
     return true;
 }
 
+// The largest t with fl(sqrt(t)) <= dist, so that t-comparisons of squared
+// distances decide as the reference's comparisons of roots do (the rounded
+// root is monotone); -1 for dist <= 0.
+float sqrt_threshold(float dist) {
+    if (!(dist > 0.0f)) return -1.0f;
+    const float big = std::numeric_limits<float>::max();
+    float t = dist * dist;
+    if (!(t <= big)) t = big;
+    while (std::sqrt(t) > dist) t = std::nextafter(t, 0.0f);
+    while (t < big && std::sqrt(std::nextafter(t, big)) <= dist) t = std::nextafter(t, big);
+    return t;
+}
+
 void set_rep_params(Rep* R, const kb_flock_params* p) {
     R->coh = p->cohesion;
     R->avo = p->avoidance;
@@ -109,6 +123,7 @@ void set_rep_params(Rep* R, const kb_flock_params* p) {
     R->mom = p->momentum;
     R->jump = p->jump;
     R->radius = p->neighbor_radius;
+    R->thr = sqrt_threshold(p->neighbor_radius);
     R->dd = (p->neighbor_radius <= 0.0f) ? -1 : as_i32(std::floor(p->neighbor_radius / R->d));
     R->qmode = p->query_mode;
     R->seed_lo = (uint32_t)p->seed;
@@ -501,6 +516,14 @@ kb_status fast_rebuild(kb_field* f, bool bump_step) {
     return KB_OK;
 }
 
+// Whether every replica suits the ring force kernels (ForceArgs::ring).
+bool ring_ok(const kb_field* f) {
+    if (!f->ids_unique || f->rn > (1u << 26)) return false;
+    for (const Rep& R : f->reps)
+        if (!R.toroidal || R.cell_wrap || !R.nowrap || R.dd > 1) return false;
+    return true;
+}
+
 kb_status enqueue_force(kb_field* f, const kb_flock_params* p) {
     ForceArgs a{};
     a.reps = f->d_rep.p;
@@ -529,6 +552,7 @@ kb_status enqueue_force(kb_field* f, const kb_flock_params* p) {
     a.self_by_slot = f->ids_unique ? 1 : 0;
     a.dense = f->dense ? 1 : 0;
     a.block_threads = f->force_block;
+    a.ring = ring_ok(f) ? 1 : 0;
     KB_CUDA(launch_flock_force(a, p->arith == KB_ARITH_STRICT, p->query_mode, f->stream));
     f->hist_counted = true;
     return KB_OK;

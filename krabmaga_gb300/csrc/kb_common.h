@@ -53,6 +53,8 @@ struct Rep {
     unsigned long long dh_magic;  // ceil(2^64 / dh): n / dh == umul64hi(n, dh_magic) for n < 2^32
     int32_t cell_wrap;      // toroidal fields: 0 clamp the query's cell range (the reference), 1 wrap it
     int32_t seg_rows;       // bags per segment of the packed segment rebin (0: the default)
+    float thr;              // the largest t with fl(sqrt(t)) <= radius (-1 when radius <= 0)
+    uint32_t _pad;
 };
 
 // ------------------------------------------------------------------ Philox

@@ -94,11 +94,17 @@ struct ForceArgs {
     // several replicas: threads per block of the block table (FORCE_BLOCKS_*;
     // 0: FORCE_THREADS), the launch shape the batch autotuner picks
     uint32_t block_threads;
+    // every replica is a torus with the clamped range, no pair
+    // straddles the seam, the ring is at most one bag wide, ids are distinct
+    // and n <= 2^26 (byte offsets of three runs in 32 bits): the ring kernels
+    int32_t ring;
 };
 constexpr int FORCE_THREADS = 256;  // the force kernel's block (one replica per block)
 // Block sizes of the force pass over packed replicas (one replica per block).
 constexpr int FORCE_BLOCK_SIZES[3] = {128, 256, 512};
 cudaError_t launch_flock_force(const ForceArgs& a, bool strict, int qmode, cudaStream_t s);
+// The same for a.ring flocks (kb_ring.cu); launch_flock_force calls it.
+cudaError_t launch_flock_ring(const ForceArgs& a, bool strict, int qmode, cudaStream_t s);
 // Whole steps of a small single-replica field in one cluster of SMALL_CTAS
 // blocks (kb_small.cu): every block loads the read buffer (st, ids, start
 // over rep.ncells bags) into its shared memory, nsteps steps run there, and

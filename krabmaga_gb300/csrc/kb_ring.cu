@@ -1,0 +1,441 @@
+// kb_ring.cu -- the force pass of flocks whose query spans at most one bag
+// around the boid's own (radius < 2 d, the usual geometry) on a torus with the
+// clamped range and distinct ids: k_flock_force's results bit for bit, for
+// less issue per candidate.  Flocks of any other kind, and the fast walk of
+// dense ones, take k_flock_force.
+//
+// The walks are written for few instructions and loads:
+//   * the boid itself stays in its list: its own terms are exact zeros (its
+//     distance is zero, and a sum that starts at +0 never becomes -0), so only
+//     its heading has to be held back, by one predicate;
+//   * fast arithmetic: x and y travel together in packed f32x2 operations (one
+//     issue slot for two IEEE results; the FMA pipe takes two cycles for it,
+//     which the fast walk has to spare and the strict one has not);
+//   * strict arithmetic: both quotients of a pair share one reciprocal
+//     (div2_rn);
+//   * exact query: distances are compared squared, with the largest square
+//     whose root is within the radius (Rep::thr), and a bag's four corners are
+//     classified from the extreme squares of its column and its row.
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <type_traits>
+
+#include "kb_common.h"
+#include "kb_device.cuh"
+#include "kb_force.cuh"
+#include "kb_launch.h"
+
+namespace kb {
+namespace {
+
+// ---- pairs of f32: packed into one register pair, or two registers
+using f32x2 = unsigned long long;
+struct f32two {
+    float x = 0.f, y = 0.f;
+};
+template <bool STRICT>
+using pair_t = typename std::conditional<STRICT, f32two, f32x2>::type;
+
+__device__ __forceinline__ void pack2(f32x2& r, float lo, float hi) {
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+}
+__device__ __forceinline__ void pack2(f32two& r, float lo, float hi) {
+    r.x = lo;
+    r.y = hi;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ void unpack2(f32two v, float& lo, float& hi) {
+    lo = v.x;
+    hi = v.y;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32two add2(f32two a, f32two b) {
+    return {__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y)};
+}
+// a - b as b * -1 + a (one rounding, the same bits): a packed subtraction is
+// two sign flips and an addition
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(b), "l"(0xBF800000BF800000ull), "l"(a));
+    return r;
+}
+__device__ __forceinline__ f32two sub2(f32two a, f32two b) {
+    return {__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y)};
+}
+// v += w unless p == my
+__device__ __forceinline__ void add2_unless(f32x2& v, f32x2 w, uint32_t p, uint32_t my) {
+    asm("{\n\t.reg .pred other;\n\tsetp.ne.u32 other, %2, %3;\n\t@other add.rn.f32x2 %0, %0, %1;\n\t}"
+        : "+l"(v)
+        : "l"(w), "r"(p), "r"(my));
+}
+__device__ __forceinline__ void add2_unless(f32two& v, f32two w, uint32_t p, uint32_t my) {
+    if (p != my) v = add2(v, w);
+}
+
+// The sums of one agent over its candidates (Acc's, in pairs).
+template <bool STRICT>
+struct Sums {
+    pair_t<STRICT> ch{}, cs{};  // cohesion, consistency
+    float ax = 0.f, ay = 0.f;   // avoidance
+    uint32_t vec = 0, count = 0;
+
+    // one candidate at d = me - o, slot p, sq its squared distance as
+    // Bird::step has it; SELF: p may be the agent's own slot `my`
+    template <bool SELF>
+    __device__ __forceinline__ void add(pair_t<STRICT> d, float sq, pair_t<STRICT> heading, uint32_t p,
+                                        uint32_t my) {
+        float dx, dy;
+        unpack2(d, dx, dy);
+        if (STRICT) {
+            const float q = __fadd_rn(__fmul_rn(sq, sq), 1.0f);
+            const float2 t = div2_rn(dx, dy, q, SELF && p == my);  // the agent itself: zeros either way
+            ax = __fadd_rn(ax, t.x);
+            ay = __fadd_rn(ay, t.y);
+        } else {
+            const float inv = rcp_approx(__fmaf_rn(sq, sq, 1.0f));
+            ax = __fmaf_rn(dx, inv, ax);
+            ay = __fmaf_rn(dy, inv, ay);
+        }
+        ch = add2(ch, d);
+        if (SELF) add2_unless(cs, heading, p, my);
+        else cs = add2(cs, heading);
+    }
+    __device__ __forceinline__ Acc<STRICT> result() const {
+        Acc<STRICT> r;
+        r.xa = ax;
+        r.ya = ay;
+        unpack2(ch, r.xc, r.yc);
+        unpack2(cs, r.xs, r.ys);
+        r.vec = vec;
+        r.count = (int)count;
+        return r;
+    }
+};
+
+// The squared distance of Bird::step's avoidance term / of the exact query.
+__device__ __forceinline__ float sq_rn(float dx, float dy) {
+    return __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+}
+template <bool STRICT>
+__device__ __forceinline__ float pair_sq(pair_t<STRICT> d) {
+    float dx, dy;
+    unpack2(d, dx, dy);
+    return STRICT ? sq_rn(dx, dy) : __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
+}
+
+template <bool STRICT>
+struct Candidate {
+    pair_t<STRICT> pos, heading;
+};
+template <bool STRICT>
+__device__ __forceinline__ Candidate<STRICT> load_candidate(const float4* q) {
+    Candidate<STRICT> c;
+    if constexpr (STRICT) {
+        const float4 v = __ldg(q);
+        c.pos = {v.x, v.y};
+        c.heading = {v.z, v.w};
+    } else {
+        const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(q));
+        c.pos = v.x;
+        c.heading = v.y;
+    }
+    return c;
+}
+
+// The candidate runs of up to three columns.
+struct Runs {
+    uint32_t s[3], e[3];
+};
+
+// Relaxed query: bags mj..Mj of columns mi..Mi (cell_range, at most 3 x 3).
+__device__ __forceinline__ void relaxed_runs(const ForceArgs& a, const Rep& R, int mi, int Mi, int mj,
+                                             int Mj, Runs& r) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        r.s[k] = r.e[k] = 0u;
+        if (mi + k <= Mi && mj <= Mj) {
+            const uint32_t c = R.cell_off + (uint32_t)(mi + k) * (uint32_t)R.dh;
+            r.e[k] = min(__ldg(a.start + c + Mj + 1), a.n);
+            r.s[k] = min(__ldg(a.start + c + mj), r.e[k]);
+        }
+    }
+}
+
+// One flat list over the three runs: a warp iterates its longest lane's total.
+// U candidates are loaded together: 1 for large flocks (issue-bound, few
+// registers), more for small ones, where too few warps hide the loads.
+template <bool STRICT, int U>
+__device__ __forceinline__ void walk_flat(const ForceArgs& a, pair_t<STRICT> me, uint32_t my,
+                                          const Runs& r, Sums<STRICT>& sums) {
+    const uint32_t P1 = r.e[0] - r.s[0], P2 = P1 + (r.e[1] - r.s[1]), T = P2 + (r.e[2] - r.s[2]);
+    const uint32_t j1 = r.s[1] - r.e[0], j2 = r.s[2] - r.e[1];
+    uint32_t p = r.s[0];
+    for (uint32_t f = 0; f < T;) {
+        Candidate<STRICT> o[U];
+        uint32_t at[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (f == P1) p += j1;
+            if (f == P2) p += j2;
+            at[u] = p;
+            if (u == 0 || f < T) o[u] = load_candidate<STRICT>(a.st + p);
+            ++p;
+            ++f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (u == 0 || f - (uint32_t)(U - u) < T) {
+                const pair_t<STRICT> d = sub2(me, o[u].pos);
+                sums.template add<true>(d, pair_sq<STRICT>(d), o[u].heading, at[u], my);
+            }
+    }
+    sums.vec = T;
+}
+
+// Long lists (dense flocks): column after column with a plain pointer, U
+// candidates loaded together; only the agent's own column is tested for the
+// agent itself.
+template <bool STRICT, bool SELF, int U>
+__device__ __forceinline__ void walk_run(const float4* st, pair_t<STRICT> me, uint32_t my, uint32_t s,
+                                         uint32_t e, Sums<STRICT>& sums) {
+    const float4* q = st + s;
+    const float4* const end = st + e;
+    uint32_t p = s;
+    auto take = [&](const Candidate<STRICT>& o, uint32_t at) {
+        const pair_t<STRICT> d = sub2(me, o.pos);
+        sums.template add<SELF>(d, pair_sq<STRICT>(d), o.heading, at, my);
+    };
+#pragma unroll 1
+    for (; end - q >= U; q += U, p += U) {
+        Candidate<STRICT> o[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) o[u] = load_candidate<STRICT>(q + u);
+#pragma unroll
+        for (int u = 0; u < U; ++u) take(o[u], p + u);
+    }
+#pragma unroll 1
+    for (; q < end; ++q, ++p) take(load_candidate<STRICT>(q), p);
+}
+
+template <bool STRICT, int U>
+__device__ __forceinline__ void walk_runs(const ForceArgs& a, pair_t<STRICT> me, uint32_t my,
+                                          const Runs& r, Sums<STRICT>& sums) {
+#pragma unroll 1
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t s = k == 0 ? r.s[0] : (k == 1 ? r.s[1] : r.s[2]);
+        const uint32_t e = k == 0 ? r.e[0] : (k == 1 ? r.e[1] : r.e[2]);
+        sums.vec += e - s;
+        if (my - s < e - s) walk_run<STRICT, true, U>(a.st, me, my, s, e, sums);
+        else walk_run<STRICT, false, U>(a.st, me, my, s, e, sums);
+    }
+}
+
+// The agent pass of the exact query (check_circle's bag rule, field_2d.rs:
+// 934-972, then the distance): the kept bags of each column as one run, with
+// the part of it whose bags count as a whole; the three runs as one flat list.
+template <bool STRICT, int U>
+__device__ __forceinline__ void walk_exact(const ForceArgs& a, const Rep& R, float4 me4, uint32_t my,
+                                           int mi, int Mi, int mj, int Mj, Sums<STRICT>& sums) {
+    pair_t<STRICT> me;
+    pack2(me, me4.x, me4.y);
+    float ymin[3], ymax[3];  // the least and greatest squared y distance of a row's corners
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const float nw = __fmul_rn((float)(mj + r), R.d);
+        const float n0 = __fsub_rn(nw, me4.y), n1 = __fsub_rn(fminf(__fadd_rn(nw, R.d), R.h), me4.y);
+        const float q0 = __fmul_rn(n0, n0), q1 = __fmul_rn(n1, n1);
+        ymin[r] = fminf(q0, q1);
+        ymax[r] = fmaxf(q0, q1);
+    }
+    uint32_t s[3], e[3], wl[3], wn[3];
+    bool apart = false;  // a skipped bag between two kept ones of a column
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        s[k] = e[k] = wl[k] = wn[k] = 0u;
+        if (mi + k > Mi || mj > Mj) continue;
+        const float nw = __fmul_rn((float)(mi + k), R.d);
+        const float n0 = __fsub_rn(nw, me4.x), n1 = __fsub_rn(fminf(__fadd_rn(nw, R.d), R.w), me4.x);
+        const float q0 = __fmul_rn(n0, n0), q1 = __fmul_rn(n1, n1);
+        const float xmin = fminf(q0, q1), xmax = fmaxf(q0, q1);
+        const uint32_t c = R.cell_off + (uint32_t)(mi + k) * (uint32_t)R.dh + (uint32_t)mj;
+        uint32_t o[4];
+#pragma unroll
+        for (int r = 3; r >= 0; --r) o[r] = min(__ldg(a.start + c + min(r, Mj - mj + 1)), a.n);
+#pragma unroll
+        for (int r = 2; r >= 0; --r) o[r] = min(o[r], o[r + 1]);
+        uint32_t keep = 0u, whole = 0u;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            if (mj + r > Mj) continue;
+            if (!(__fadd_rn(xmin, ymin[r]) > R.thr)) keep |= 1u << r;
+            if (__fadd_rn(xmax, ymax[r]) <= R.thr) whole |= 1u << r;
+        }
+        apart |= keep == 5u || whole == 5u;
+        if (keep) {
+            s[k] = (keep & 1u) ? o[0] : ((keep & 2u) ? o[1] : o[2]);
+            e[k] = (keep & 4u) ? o[3] : ((keep & 2u) ? o[2] : o[1]);
+        }
+        if (whole) {
+            wl[k] = (whole & 1u) ? o[0] : ((whole & 2u) ? o[1] : o[2]);
+            wn[k] = ((whole & 4u) ? o[3] : ((whole & 2u) ? o[2] : o[1])) - wl[k];
+        }
+    }
+    auto take = [&](const Candidate<STRICT>& o, uint32_t p, bool all) {
+        const pair_t<STRICT> d = sub2(me, o.pos);
+        float dx, dy;
+        unpack2(d, dx, dy);
+        const float sq = sq_rn(dx, dy);
+        if (all || sq <= R.thr) {
+            sums.template add<true>(d, STRICT ? sq : pair_sq<STRICT>(d), o.heading, p, my);
+            sums.vec += 1u;
+            sums.count += p != my ? 1u : 0u;
+        }
+    };
+    if (apart) {  // rounding at a bag's edge: bag by bag
+#pragma unroll 1
+        for (int k = 0; mi + k <= Mi; ++k) {
+#pragma unroll 1
+            for (int r = 0; mj + r <= Mj; ++r) {
+                const int check = check_circle(mi + k, mj + r, R, me4.x, me4.y, R.radius);
+                if (check == -1) continue;
+                const uint32_t c = R.cell_off + (uint32_t)(mi + k) * (uint32_t)R.dh + (uint32_t)(mj + r);
+                const uint32_t end = min(__ldg(a.start + c + 1), a.n);
+#pragma unroll 1
+                for (uint32_t p = min(__ldg(a.start + c), end); p < end; ++p)
+                    take(load_candidate<STRICT>(a.st + p), p, check == 1);
+            }
+        }
+        return;
+    }
+    const uint32_t P1 = e[0] - s[0], P2 = P1 + (e[1] - s[1]), T = P2 + (e[2] - s[2]);
+    uint32_t p = s[0], w0 = wl[0], w1 = wn[0];
+    for (uint32_t f = 0; f < T;) {
+        Candidate<STRICT> o[U];
+        uint32_t at[U];
+        bool all[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (f == P1) { p = s[1]; w0 = wl[1]; w1 = wn[1]; }
+            if (f == P2) { p = s[2]; w0 = wl[2]; w1 = wn[2]; }
+            at[u] = p;
+            all[u] = p - w0 < w1;
+            if (u == 0 || f < T) o[u] = load_candidate<STRICT>(a.st + p);
+            ++p;
+            ++f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (u == 0 || f - (uint32_t)(U - u) < T) take(o[u], at[u], all[u]);
+    }
+}
+
+// How the relaxed query's lists are walked: as one flat list, run by run, or
+// by the warp's own longest list (packed replicas, whose flocks differ).
+enum Walk { WALK_FLAT, WALK_RUNS, WALK_VOTE };
+constexpr uint32_t VOTE_LIST = 32;
+
+template <bool STRICT, bool EXACT, Walk WALK, int U>
+__device__ __forceinline__ void ring_body(const ForceArgs& a, const Rep& R, uint32_t i) {
+    const unsigned long long step = *a.step;
+    const float4 me = __ldg(a.st + i);
+    const uint32_t my_id = __ldg(a.ids + i);
+    Sums<STRICT> sums;
+    int mi, Mi, mj, Mj;
+    if (cell_range(R, me.x, me.y, R.dd, &mi, &Mi, &mj, &Mj)) {
+        if (EXACT) {
+            walk_exact<STRICT, U>(a, R, me, i, mi, Mi, mj, Mj, sums);
+        } else {
+            pair_t<STRICT> mxy;
+            pack2(mxy, me.x, me.y);
+            Runs r;
+            relaxed_runs(a, R, mi, Mi, mj, Mj, r);
+            const bool self_in = (i - r.s[0] < r.e[0] - r.s[0]) || (i - r.s[1] < r.e[1] - r.s[1]) ||
+                                 (i - r.s[2] < r.e[2] - r.s[2]);
+            const uint32_t T = (r.e[0] - r.s[0]) + (r.e[1] - r.s[1]) + (r.e[2] - r.s[2]);
+            if (WALK == WALK_RUNS || (WALK == WALK_VOTE && __any_sync(__activemask(), T >= VOTE_LIST)))
+                walk_runs<STRICT, 4>(a, mxy, i, r, sums);
+            else
+                walk_flat<STRICT, U>(a, mxy, i, r, sums);
+            sums.count = sums.vec - (self_in ? 1u : 0u);
+        }
+    }
+    force_finish<STRICT, WALK != WALK_RUNS>(a, R, i, me, my_id, step, sums.result());
+}
+
+template <bool STRICT, bool EXACT, Walk WALK, bool MULTI, int U, int BT, int MINB>
+__global__ void __launch_bounds__(BT, MINB) k_flock_ring(ForceArgs a) {
+    pdl_enter();
+    if (MULTI) {
+        // one replica per block: its record is read once into shared memory
+        __shared__ Rep sR;
+        const uint2 e = a.blk[blockIdx.x];
+        load_rep_shared(&sR, a.reps + e.x);
+        __syncthreads();
+        const uint32_t k = e.y + threadIdx.x;
+        if (k >= sR.boid_off + sR.nboids) return;
+        ring_body<STRICT, EXACT, WALK, U>(a, sR, k);
+    } else {
+        const uint32_t i = blockIdx.x * BT + threadIdx.x;
+        if (i >= a.n) return;
+        ring_body<STRICT, EXACT, WALK, U>(a, a.rep0, i);
+    }
+}
+
+// Launch shapes, measured on GB300 (us per step, density 0.025 unless said):
+//   * up to SMALL_N boids the pass is bound by latency: 128-thread blocks of up
+//     to 64 registers, the strict walk two candidates at a time (20k 8.2, 262k
+//     15.3; the throughput shape 8.3 and 16.8; 65k strict 10.8 with two at a
+//     time, 11.4 with one; fast 9.0 with one, 9.7 with two);
+//   * above it by issue: fast 32 registers and all 64 warps (1M 40.6; 40 and 48
+//     registers 42.1), strict 48 registers (1M 54.4; 40 and 64 registers 56 to
+//     58).  k_flock_force: 42.6 and 61.7;
+//   * exact query, 65k strict: 12.4 against 30 for k_flock_force;
+//   * long lists, strict (131k clustered): 115 against 156 with 4 candidates
+//     loaded together and 64 registers (2 and 48: 128).  The fast walk of long
+//     lists is bound by L1, whose 16-byte loads return 512 B a warp for one
+//     candidate (70 % of its wavefronts): k_flock_force has it at the same speed.
+//     Two boids of a bag per thread, sharing the loads, halve that traffic but
+//     leave lanes idle where bags end: 224 against 228 us, not kept;
+//   * packed replicas: 48 registers and the walk by vote.  64 replicas, steps
+//     0-100 / 400-500 (condensed flocks): 74.8 / 93.4 us, flat walk 78.7 / 108.6,
+//     k_flock_force 78.6 / 106.0; from 24 or 40 candidates the same, from 64
+//     79.9 / 98.5; two or eight candidates together 77.9 / 100.0, 78.1 / 94.8.
+constexpr uint32_t SMALL_N = 400000;
+
+template <bool STRICT, bool EXACT>
+cudaError_t launch_ring(const ForceArgs& a, cudaStream_t s) {
+    // resident blocks of 256 threads per SM
+    constexpr int MINB = EXACT ? 4 : (STRICT ? 5 : 8);
+    constexpr int MM = EXACT ? 4 : 5;  // packed replicas
+    if (a.nrep > 1) {
+        if (a.block_threads == 128)
+            return launch_pdl(k_flock_ring<STRICT, EXACT, WALK_VOTE, true, 1, 128, 2 * MM>, a.nblk, 128, s, a);
+        if (a.block_threads == 512)
+            return launch_pdl(k_flock_ring<STRICT, EXACT, WALK_VOTE, true, 1, 512, MM / 2>, a.nblk, 512, s, a);
+        return launch_pdl(k_flock_ring<STRICT, EXACT, WALK_VOTE, true, 1, 256, MM>, a.nblk, 256, s, a);
+    }
+    const unsigned g = grid_for(a.n, 128);
+    if constexpr (STRICT && !EXACT)
+        if (a.dense) return launch_pdl(k_flock_ring<true, false, WALK_RUNS, false, 1, 128, 8>, g, 128, s, a);
+    if (a.n <= SMALL_N)
+        return launch_pdl(k_flock_ring<STRICT, EXACT, WALK_FLAT, false, STRICT ? 2 : 1, 128, 8>, g, 128, s, a);
+    return launch_pdl(k_flock_ring<STRICT, EXACT, WALK_FLAT, false, 1, 128, 2 * MINB>, g, 128, s, a);
+}
+
+}  // namespace
+
+cudaError_t launch_flock_ring(const ForceArgs& a, bool strict, int qmode, cudaStream_t s) {
+    if (a.n == 0) return cudaSuccess;
+    if (a.nrep > 1 && a.blk == nullptr) return cudaErrorInvalidValue;
+    if (qmode == 0) return strict ? launch_ring<true, false>(a, s) : launch_ring<false, false>(a, s);
+    return strict ? launch_ring<true, true>(a, s) : launch_ring<false, true>(a, s);
+}
+
+}  // namespace kb
