@@ -485,7 +485,15 @@ kb_status general_rebuild(kb_field* f, bool counted) {
     return KB_OK;
 }
 
-kb_status fast_rebuild(kb_field* f, bool bump_step) {
+// Whether the ranked rebin takes a write list whose moves the source lines may
+// not cover (long moves, objects set apart from their own positions).
+bool rank_any(const kb_field* f) {
+    return f->slots_kept && f->reps.size() == 1 && f->rn <= RANK_ANY_MAX;
+}
+
+// The rebuild of a whole force pass: stencil, by segments or ranks, or any
+// moves by ranks (stencil false; see rank_any).
+kb_status fast_rebuild(kb_field* f, bool bump_step, bool stencil) {
     cudaStream_t s = f->stream;
     const int nxt = 1 - f->cur;
     KB_CUDA(launch_scan(f->hist.p, f->start[nxt].p, f->ncells_total, f->scan_ctl.p, f->tstate.p, f->err.p, true, s,
@@ -511,17 +519,24 @@ kb_status fast_rebuild(kb_field* f, bool bump_step) {
     a.err = f->err.p;
     a.n = f->rn;
     a.slots = f->slots_kept ? f->slots.p : nullptr;
+    a.any_move = stencil ? 0 : 1;
     KB_CUDA(launch_rebin(a, s));
     f->cur = nxt;
     return KB_OK;
 }
 
-// Whether every replica suits the ring force kernels (ForceArgs::ring).
-bool ring_ok(const kb_field* f) {
+// Whether every replica suits the ring force kernels (ForceArgs::ring), or a
+// small plain field the warp-per-boid one (ForceArgs::wide).
+bool ring_ok(const kb_field* f, bool* wide) {
+    *wide = false;
     if (!f->ids_unique || f->rn > (1u << 26)) return false;
-    for (const Rep& R : f->reps)
-        if (!R.toroidal || R.cell_wrap || !R.nowrap || R.dd > 1) return false;
-    return true;
+    bool one = true;
+    for (const Rep& R : f->reps) {
+        if (!R.toroidal || R.cell_wrap || !R.nowrap) return false;
+        one = one && R.dd <= 1;
+    }
+    *wide = !one && f->reps.size() == 1 && f->rn <= wide_max(f->reps[0].dd, f->reps[0].qmode);
+    return one;
 }
 
 kb_status enqueue_force(kb_field* f, const kb_flock_params* p) {
@@ -552,7 +567,9 @@ kb_status enqueue_force(kb_field* f, const kb_flock_params* p) {
     a.self_by_slot = f->ids_unique ? 1 : 0;
     a.dense = f->dense ? 1 : 0;
     a.block_threads = f->force_block;
-    a.ring = ring_ok(f) ? 1 : 0;
+    bool wide = false;
+    a.ring = ring_ok(f, &wide) ? 1 : 0;
+    a.wide = wide && !f->dense ? 1 : 0;
     KB_CUDA(launch_flock_force(a, p->arith == KB_ARITH_STRICT, p->query_mode, f->stream));
     f->hist_counted = true;
     return KB_OK;
@@ -935,7 +952,8 @@ kb_status field_lazy_update(kb_field* f) {
     // field_2d.rs:905-921: the first swap fixes nagents' density estimate.
     if (!f->density_check) f->density_check = true;
     if (f->w_from_compute && !f->w_has_dead) {
-        if (all_fast_rebin_ok(f) && f->layout_is_positions) st = fast_rebuild(f, false);
+        const bool stencil = all_fast_rebin_ok(f) && f->layout_is_positions;
+        if (stencil || rank_any(f)) st = fast_rebuild(f, false, stencil);
         else st = general_rebuild(f, true);
         if (st) return st;
         f->rn = f->wn;
@@ -2122,11 +2140,12 @@ kb_status enqueue_steps(kb_field* f, const kb_flock_params* p, uint32_t nsteps, 
         if (t >= 0) KB_CUDA(cudaEventRecord(f->kt_pending[t].ev[1], f->stream));
         f->wn = f->rn;
         f->kt_cur = t;
-        st = fast ? fast_rebuild(f, true) : general_rebuild(f, true);
+        const bool ranked = !fast && rank_any(f);
+        st = fast || ranked ? fast_rebuild(f, true, fast) : general_rebuild(f, true);
         f->kt_cur = -1;
         if (st) return st;
         if (t >= 0) KB_CUDA(cudaEventRecord(f->kt_pending[t].ev[3], f->stream));
-        if (!fast) KB_CUDA(launch_add_u64(f->dstep.p, 1ull, f->stream));
+        if (!fast && !ranked) KB_CUDA(launch_add_u64(f->dstep.p, 1ull, f->stream));
         f->wn = 0;
     }
     return KB_OK;

@@ -1057,7 +1057,9 @@ __device__ __noinline__ void place_by_lines(const RebinArgs& a, bool over, uint3
                 rank += mine ? __popc(d >= 32u ? m : m & ((1u << d) - 1u)) : 0;
             }
         };
-        if (X > 0 && X < R.seam && Y > 0 && Y < R.seam) {
+        if (a.any_move) {
+            count(0u, a.n);
+        } else if (X > 0 && X < R.seam && Y > 0 && Y < R.seam) {
 #pragma unroll 1
             for (int q = -1; q <= 1; ++q) {
                 const uint32_t c = R.cell_off + (uint32_t)(X + q) * (uint32_t)R.dh + (uint32_t)Y;
@@ -1609,6 +1611,7 @@ cudaError_t launch_flock_force(const ForceArgs& a, bool strict, int qmode, cudaS
     if (a.n == 0) return cudaSuccess;
     const bool multi = a.nrep > 1;
     if (multi && a.blk == nullptr) return cudaErrorInvalidValue;
+    if (a.wide) return launch_flock_wide(a, strict, qmode, s);
     if (a.ring && (strict || qmode != 0 || !a.dense)) return launch_flock_ring(a, strict, qmode, s);
     const unsigned g = multi ? a.nblk : grid_for(a.n, KB_FORCE_THREADS);
 #define KB_FORCE(S, Q, MU)                                                                      \

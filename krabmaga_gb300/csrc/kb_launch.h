@@ -98,13 +98,25 @@ struct ForceArgs {
     // straddles the seam, the ring is at most one bag wide, ids are distinct
     // and n <= 2^26 (byte offsets of three runs in 32 bits): the ring kernels
     int32_t ring;
+    // the same with a wider ring, one replica of at most wide_max boids: the
+    // warp-per-boid kernel
+    int32_t wide;
 };
+// Up to how many boids the warp-per-boid kernel is the faster one: it gives a
+// boid 32 lanes, k_flock_force gives it one and waits for its columns in turn.
+// Measured (us per step, warp / thread per boid): 7 columns 8k 12.0 / 16.9, 20k
+// 18.2 / 18.0, 32k 24.7 / 18.4; 41 columns 1k 10.1 / 47, 20k 31 / 59; exact, 7
+// columns 8k 14.8 / 64.7, 41 columns 20k 45 / 764 (a corner rule per bag).
+inline uint32_t wide_max(int32_t dd, int32_t qmode) {
+    return qmode != 0 ? 262144u : (2 * dd + 1 >= 16 ? 32768u : 16384u);
+}
 constexpr int FORCE_THREADS = 256;  // the force kernel's block (one replica per block)
 // Block sizes of the force pass over packed replicas (one replica per block).
 constexpr int FORCE_BLOCK_SIZES[3] = {128, 256, 512};
 cudaError_t launch_flock_force(const ForceArgs& a, bool strict, int qmode, cudaStream_t s);
 // The same for a.ring flocks (kb_ring.cu); launch_flock_force calls it.
 cudaError_t launch_flock_ring(const ForceArgs& a, bool strict, int qmode, cudaStream_t s);
+cudaError_t launch_flock_wide(const ForceArgs& a, bool strict, int qmode, cudaStream_t s);
 // Whole steps of a small single-replica field in one cluster of SMALL_CTAS
 // blocks (kb_small.cu): every block loads the read buffer (st, ids, start
 // over rep.ncells bags) into its shared memory, nsteps steps run there, and
@@ -163,6 +175,9 @@ struct RebinArgs {
     uint32_t* err;
     uint32_t n;  // records (every slot index is below it)
     const uint32_t* slots;  // the force pass's arrival slots: the ranked rebin (nullptr: by segments)
+    // moves may cross more than one bag: a fuller bag's arrivals are counted in
+    // the whole list (ranked rebin only, up to RANK_ANY_MAX records)
+    int32_t any_move;
 };
 // Arrivals per bag whose write-list slots the force pass records: the first
 // four of every bag in one array of 16 B per bag, the next eight in a second
@@ -171,6 +186,10 @@ struct RebinArgs {
 // 44.6 us for a row of 4: the step's working set is near the L2's size.)
 constexpr uint32_t RANK_ROW = 4, RANK_ROW2 = 8;
 constexpr uint32_t RANK_SLOTS = RANK_ROW + RANK_ROW2;
+// Records up to which the ranked rebin takes flocks whose moves the source
+// lines do not cover: a warp then reads the whole list for each of its fuller
+// bags (about 10 us at this length).
+constexpr uint32_t RANK_ANY_MAX = 32768;
 // Bag matrices up to this many bags carry the arrival slots (48 B per bag).
 constexpr uint32_t RANK_MAX_CELLS = 1u << 26;
 // Bag segments of the segment rebin: SEG_ROWS consecutive bags of one column.
