@@ -189,12 +189,12 @@ kb_status grow(kb_field* f, uint32_t need) {
     if (need > nc) return fail(KB_ERR_ARG, "object count exceeds 2^32-16");
     const uint32_t c = (uint32_t)nc;
     DevBuf<float4> rst, wst, tst;
-    DevBuf<uint32_t> rid, wid, wkey, tid, tsrc, rkey, tkey;
+    DevBuf<uint32_t> rid, wid, wkey, tid, tsrc;
     DevBuf<uint8_t> wdead;
     cudaError_t e;
     if ((e = rst.alloc(c)) || (e = wst.alloc(c)) || (e = tst.alloc(c)) || (e = rid.alloc(c)) ||
         (e = wid.alloc(c)) || (e = wkey.alloc(c)) || (e = tid.alloc(c)) || (e = tsrc.alloc(c)) ||
-        (e = wdead.alloc(c)) || (e = rkey.alloc(c)) || (e = tkey.alloc(c)))
+        (e = wdead.alloc(c)))
         return cuda_fail(e, "growing object storage");
     // no removal marks outside the live write list (they are cleared as consumed)
     KB_CUDA(cudaMemsetAsync(wdead.p, 0, c, f->stream));
@@ -212,7 +212,7 @@ kb_status grow(kb_field* f, uint32_t need) {
     f->rst.swap(rst); f->wst.swap(wst); f->tst.swap(tst);
     f->rid.swap(rid); f->wid.swap(wid); f->wkey.swap(wkey);
     f->tid.swap(tid); f->tsrc.swap(tsrc); f->wdead.swap(wdead);
-    f->rkey.swap(rkey); f->tkey.swap(tkey);
+    f->rkey.release(); f->tkey.release();  // the tiled steps' own, made by fused_prepare
     f->cap = c;
     f->drop_graphs();
     return KB_OK;
@@ -285,22 +285,27 @@ void set_dense(kb_field* f, bool d) {
     f->dense = d;
 }
 
+// The field's page of pinned words, made on first use (nullptr: none to be had).
+unsigned long long* pinned_page(kb_field* f) {
+    if (!f->occ_host && cudaMallocHost(&f->occ_host, sizeof(unsigned long long) * PIN_WORDS) != cudaSuccess) {
+        cudaGetLastError();
+        f->occ_host = nullptr;
+    }
+    return f->occ_host;
+}
+
 // Enqueue a measurement of the read buffer into the pinned word (no wait).
 kb_status occ_enqueue(kb_field* f) {
     if (f->reps.size() != 1 || f->virt) return KB_OK;
-    if (!f->occ_host) {
-        if (cudaMallocHost(&f->occ_host, sizeof(unsigned long long)) != cudaSuccess) {
-            cudaGetLastError();
-            f->occ_host = nullptr;
-            return KB_OK;  // no measurement: the flag stays as it is
-        }
+    if (!pinned_page(f)) return KB_OK;  // no measurement: the flag stays as it is
+    if (!f->occ_ev) {
         cudaError_t e = f->occ_dev.alloc(1);
         if (!e) e = cudaEventCreateWithFlags(&f->occ_ev, cudaEventDisableTiming);
         if (e) return cuda_fail(e, "occupancy measurement");
     }
     KB_CUDA(cudaMemsetAsync(f->occ_dev.p, 0, sizeof(unsigned long long), f->stream));
     KB_CUDA(launch_occupancy_sq(f->start[f->cur].p, f->ncells_total, f->occ_dev.p, f->stream));
-    KB_CUDA(cudaMemcpyAsync(f->occ_host, f->occ_dev.p, sizeof(unsigned long long),
+    KB_CUDA(cudaMemcpyAsync(f->occ_host + PIN_OCC, f->occ_dev.p, sizeof(unsigned long long),
                             cudaMemcpyDeviceToHost, f->stream));
     KB_CUDA(cudaEventRecord(f->occ_ev, f->stream));
     f->occ_pending = true;
@@ -320,7 +325,7 @@ void occ_poll(kb_field* f) {
         return;
     }
     f->occ_pending = false;
-    set_dense(f, dense_from(*f->occ_host, f->occ_n));
+    set_dense(f, dense_from(f->occ_host[PIN_OCC], f->occ_n));
 }
 
 // Whole steps in one thread block (kb_small.cu): a plain field small enough
@@ -388,6 +393,13 @@ kb_status flush_pending(kb_field* f) {
 }
 
 kb_status read_u32(kb_field* f, const uint32_t* dptr, uint32_t* out) {
+    if (f->occ_host) {  // through pinned memory: no staging copy
+        uint32_t* w = reinterpret_cast<uint32_t*>(f->occ_host + PIN_WORD);
+        KB_CUDA(cudaMemcpyAsync(w, dptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, f->stream));
+        KB_CUDA(cudaStreamSynchronize(f->stream));
+        *out = *w;
+        return KB_OK;
+    }
     KB_CUDA(cudaMemcpyAsync(out, dptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, f->stream));
     KB_CUDA(cudaStreamSynchronize(f->stream));
     return KB_OK;
@@ -465,22 +477,31 @@ uint32_t* rank_slots(const kb_field* f) {
     return f->dense && f->reps.size() == 1 ? nullptr : f->slots.p;
 }
 
-// The general stable sort: write list -> read buffer.  hist already holds
-// the key counts when counted == true.
-kb_status general_rebuild(kb_field* f, bool counted) {
+// The general stable sort: write list -> read buffer (any list: counted here).
+kb_status general_rebuild(kb_field* f) {
     cudaStream_t s = f->stream;
     const int nxt = 1 - f->cur;
-    if (!counted) {
-        // a force pass may have counted the list before it was edited
-        if (f->hist_counted)
-            KB_CUDA(cudaMemsetAsync(f->hist.p, 0, sizeof(uint32_t) * f->ncells_total, s));
-        KB_CUDA(launch_hist_list(f->wkey.p, f->wdead.p, f->wn, f->hist.p, s));
-    }
+    // a force pass may have counted the list
+    if (f->hist_counted) KB_CUDA(cudaMemsetAsync(f->hist.p, 0, sizeof(uint32_t) * f->ncells_total, s));
     f->hist_counted = false;  // the scan below zeroes it
+    f->slots_kept = false;
+    KB_CUDA(launch_count_list(f->wkey.p, f->wdead.p, f->wn, f->hist.p, f->slots.p, f->ncells_total, f->tid.p, s));
     KB_CUDA(launch_scan(f->hist.p, f->start[nxt].p, f->ncells_total, f->scan_ctl.p, f->tstate.p, f->err.p, true, s,
                         scan_wait(f)));
-    KB_CUDA(launch_scatter_list(f->wkey.p, f->wdead.p, f->wst.p, f->wid.p, f->wn, f->start[nxt].p, f->cursor.p, f->tst.p, f->tid.p, f->tsrc.p, s));
-    KB_CUDA(launch_canon(f->start[nxt].p, f->ncells_total, f->tst.p, f->tid.p, f->tsrc.p, f->cursor.p, f->rst.p, f->rid.p, s));
+    PlaceArgs a{};
+    a.key = f->wkey.p;
+    a.dead = f->wdead.p;
+    a.st = f->wst.p;
+    a.ids = f->wid.p;
+    a.n = f->wn;
+    a.arrival = f->tid.p;
+    a.start = f->start[nxt].p;
+    a.ncells = f->ncells_total;
+    a.slots = f->slots.p;
+    a.order = f->tsrc.p;
+    a.s_st = f->rst.p;
+    a.s_ids = f->rid.p;
+    KB_CUDA(launch_place_list(a, s));
     f->cur = nxt;
     return KB_OK;
 }
@@ -657,6 +678,12 @@ kb_status fused_prepare(kb_field* f, const kb_flock_params* p) {
     const int strict = p->arith == KB_ARITH_STRICT ? 1 : 0;
     int dd = 0;
     for (const Rep& R : f->reps) dd = std::max(dd, R.dd);
+    if (f->rkey.n < f->cap || f->tkey.n < f->cap) {
+        cudaError_t e = f->rkey.alloc(f->cap);
+        if (!e) e = f->tkey.alloc(f->cap);
+        if (e) return cuda_fail(e, "tiled step keys");
+        f->drop_graphs();
+    }
     if (F.ready && F.n == f->rn && F.strict == strict && F.qmode == p->query_mode && F.dd == dd)
         return KB_OK;
     F.ready = false;
@@ -919,12 +946,8 @@ void set_ids_unique(kb_field* f, bool u) {
     f->ids_unique = u;
 }
 
-// Whether the read buffer's ids are distinct within each replica.
-kb_status check_unique_ids(kb_field* f) {
-    if (f->rn == 0) {
-        set_ids_unique(f, true);
-        return KB_OK;
-    }
+// Distinct ids by hashing, for ids that are not below their replica's boid count.
+kb_status check_unique_hashed(kb_field* f) {
     uint64_t cap = 1024;
     while (cap < 2ull * f->rn) cap <<= 1;
     if (cap > 0x80000000ull) {
@@ -935,13 +958,43 @@ kb_status check_unique_ids(kb_field* f) {
         cudaError_t e = f->dup_tab.alloc(cap);
         if (e) return cuda_fail(e, "id check table");
     }
-    if (kb_status st = upload_rep(f)) return st;
     KB_CUDA(cudaMemsetAsync(f->small.p, 0, sizeof(uint32_t), f->stream));
     KB_CUDA(launch_dup_check(f->d_rep.p, nrep(f), f->rid.p, f->rn, f->dup_tab.p, (uint32_t)cap,
                              f->small.p, f->stream));
     uint32_t dup = 0;
     if (kb_status st = read_u32(f, f->small.p, &dup)) return st;
     set_ids_unique(f, dup == 0);
+    return KB_OK;
+}
+
+// After a general rebuild of `most` records at most: how many are stored, how
+// dense a plain field is, and whether ids are distinct within each replica, in
+// one launch and one read (ids below their replica's boid count, the usual
+// ones, are marked in a bitmap; others are compared by hashing after it).
+kb_status load_facts(kb_field* f, uint32_t most) {
+    const bool plain = f->reps.size() == 1;
+    const size_t words = (size_t)most / 32u + 1u;
+    cudaError_t e = cudaSuccess;
+    if (f->id_bits.n < words) e = f->id_bits.alloc(words);
+    if (!e && f->facts.n < 3) e = f->facts.alloc(3);
+    if (e) return cuda_fail(e, "load facts");
+    unsigned long long local[3];
+    unsigned long long* r = pinned_page(f) ? f->occ_host + PIN_FACTS : local;
+    KB_CUDA(cudaMemsetAsync(f->id_bits.p, 0, sizeof(uint32_t) * words, f->stream));
+    KB_CUDA(cudaMemsetAsync(f->facts.p, 0, sizeof(unsigned long long) * 3, f->stream));
+    KB_CUDA(launch_load_facts(f->d_rep.p, nrep(f), most, f->rid.p, f->start[f->cur].p,
+                              plain ? f->ncells_total : 0u, f->start[f->cur].p + f->ncells_total, most,
+                              f->id_bits.p, f->facts.p, f->stream));
+    KB_CUDA(cudaMemcpyAsync(r, f->facts.p, sizeof(unsigned long long) * 3, cudaMemcpyDeviceToHost, f->stream));
+    KB_CUDA(cudaStreamSynchronize(f->stream));
+    f->rn = (uint32_t)r[2];
+    if (plain) {
+        f->occ_pending = false;
+        f->steps_since_occ = 0;
+        set_dense(f, dense_from(r[0], f->rn));
+    }
+    if ((r[1] & 3ull) == 2ull) return check_unique_hashed(f);
+    set_ids_unique(f, r[1] == 0ull);
     return KB_OK;
 }
 
@@ -954,24 +1007,14 @@ kb_status field_lazy_update(kb_field* f) {
     if (f->w_from_compute && !f->w_has_dead) {
         const bool stencil = all_fast_rebin_ok(f) && f->layout_is_positions;
         if (stencil || rank_any(f)) st = fast_rebuild(f, false, stencil);
-        else st = general_rebuild(f, true);
+        else st = general_rebuild(f);
         if (st) return st;
         f->rn = f->wn;
         f->layout_is_positions = true;
     } else {
-        st = general_rebuild(f, false);
+        st = general_rebuild(f);
         if (st) return st;
-        if ((st = occ_enqueue(f))) return st;  // completes with the read below
-        uint32_t total = 0;
-        st = read_u32(f, f->start[f->cur].p + f->ncells_total, &total);
-        if (st) return st;
-        f->rn = total;
-        if (f->occ_pending) {
-            f->occ_n = total;
-            occ_poll(f);
-        }
-        // the id multiset may have changed
-        if ((st = check_unique_ids(f))) return st;
+        if ((st = load_facts(f, f->wn))) return st;
     }
     // the removal marks are consumed: the next write list starts with none
     if (f->w_has_dead && f->wn) KB_CUDA(cudaMemsetAsync(f->wdead.p, 0, f->wn, f->stream));
@@ -1028,7 +1071,6 @@ kb_status field_new(int device, const std::vector<Rep>& reps, bool is_batch, uin
     if (!e) e = f->start[0].alloc((size_t)nc + 1);
     if (!e) e = f->start[1].alloc((size_t)nc + 1);
     if (!e) e = f->hist.alloc(nc);
-    if (!e) e = f->cursor.alloc(nc);
     if (!e && nc <= RANK_MAX_CELLS) e = f->slots.alloc((size_t)nc * RANK_SLOTS);
     if (!e) e = f->scan_ctl.alloc(1);
     if (!e) e = f->aux_ctl.alloc(1);
@@ -1039,7 +1081,6 @@ kb_status field_new(int device, const std::vector<Rep>& reps, bool is_batch, uin
     if (!e) e = cudaMemsetAsync(f->start[0].p, 0, sizeof(uint32_t) * ((size_t)nc + 1), f->stream);
     if (!e) e = cudaMemsetAsync(f->start[1].p, 0, sizeof(uint32_t) * ((size_t)nc + 1), f->stream);
     if (!e) e = cudaMemsetAsync(f->hist.p, 0, sizeof(uint32_t) * nc, f->stream);
-    if (!e) e = cudaMemsetAsync(f->cursor.p, 0, sizeof(uint32_t) * nc, f->stream);
     if (!e) e = cudaMemsetAsync(f->scan_ctl.p, 0, sizeof(ScanCtl), f->stream);
     if (!e) e = cudaMemsetAsync(f->aux_ctl.p, 0, sizeof(ScanCtl), f->stream);
     if (!e) e = cudaMemsetAsync(f->tstate.p, 0, sizeof(unsigned long long) * nt, f->stream);
@@ -1073,23 +1114,21 @@ kb_status grow_cells(kb_field* f, uint64_t need) {
     if (need > 0xF0000000ull) return fail(KB_ERR_ARG, "bag matrix too large");
     const uint32_t nc = (uint32_t)std::min<uint64_t>(0xF0000000ull, std::max<uint64_t>(need, 2ull * f->cells_cap));
     const uint32_t nt = scan_state_words(nc);
-    DevBuf<uint32_t> s0, s1, hist, cursor, slots;
+    DevBuf<uint32_t> s0, s1, hist, slots;
     DevBuf<unsigned long long> ts;
     cudaError_t e;
     if ((e = s0.alloc((size_t)nc + 1)) || (e = s1.alloc((size_t)nc + 1)) || (e = hist.alloc(nc)) ||
-        (e = cursor.alloc(nc)) || (e = ts.alloc(nt)) ||
+        (e = ts.alloc(nt)) ||
         (nc <= RANK_MAX_CELLS && (e = slots.alloc((size_t)nc * RANK_SLOTS))))
         return cuda_fail(e, "growing the bag arrays");
     KB_CUDA(cudaMemsetAsync(s0.p, 0, sizeof(uint32_t) * ((size_t)nc + 1), f->stream));
     KB_CUDA(cudaMemsetAsync(s1.p, 0, sizeof(uint32_t) * ((size_t)nc + 1), f->stream));
     KB_CUDA(cudaMemsetAsync(hist.p, 0, sizeof(uint32_t) * nc, f->stream));
-    KB_CUDA(cudaMemsetAsync(cursor.p, 0, sizeof(uint32_t) * nc, f->stream));
     KB_CUDA(cudaMemsetAsync(ts.p, 0, sizeof(unsigned long long) * nt, f->stream));
     KB_CUDA(cudaStreamSynchronize(f->stream));
     f->start[0].swap(s0);
     f->start[1].swap(s1);
     f->hist.swap(hist);
-    f->cursor.swap(cursor);
     f->slots.swap(slots);
     f->tstate.swap(ts);
     f->cells_cap = nc;
@@ -2023,7 +2062,7 @@ kb_status kb_flock_next_states_device(kb_field* f, const kb_flock_params* p, uin
     a.step = f->dstep.p;
     a.out_st = reinterpret_cast<float4*>(out_dev);
     a.out_ids = f->tid.p;
-    a.out_key = f->tkey.p;
+    a.out_key = f->tsrc.p;
     a.hist = f->spare_hist.p;
     a.err = f->err.p;
     KB_CUDA(launch_flock_agents(a, reinterpret_cast<const float4*>(states_dev), ids_dev, m,
@@ -2141,7 +2180,7 @@ kb_status enqueue_steps(kb_field* f, const kb_flock_params* p, uint32_t nsteps, 
         f->wn = f->rn;
         f->kt_cur = t;
         const bool ranked = !fast && rank_any(f);
-        st = fast || ranked ? fast_rebuild(f, true, fast) : general_rebuild(f, true);
+        st = fast || ranked ? fast_rebuild(f, true, fast) : general_rebuild(f);
         f->kt_cur = -1;
         if (st) return st;
         if (t >= 0) KB_CUDA(cudaEventRecord(f->kt_pending[t].ev[3], f->stream));

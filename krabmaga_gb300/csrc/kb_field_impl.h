@@ -19,6 +19,10 @@
 
 using namespace kb;
 
+// Words of a field's pinned page: the occupancy measurement of running steps, the
+// three results of a load, a word read back.
+enum { PIN_OCC = 0, PIN_FACTS = 1, PIN_WORD = 4, PIN_WORDS = 8 };
+
 struct kb_field {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -50,7 +54,7 @@ struct kb_field {
     std::vector<uint32_t> p_id, p_key;
     bool p_loc_differs = false;
     // step temporaries
-    DevBuf<uint32_t> hist, cursor, tid, tsrc, rkey, tkey;
+    DevBuf<uint32_t> hist, tid, tsrc, rkey, tkey;  // rkey, tkey: the tiled steps' only
     // arrival slots of the ranked rebin, RANK_SLOTS per bag (empty above
     // RANK_MAX_CELLS bags: those fields rebin by segments)
     DevBuf<uint32_t> slots;
@@ -59,7 +63,9 @@ struct kb_field {
     // Every replica's ids are distinct in the read buffer (checked on the
     // device after each general rebuild; the step paths keep the id multiset)
     bool ids_unique = false;
-    DevBuf<unsigned long long> dup_tab;
+    DevBuf<unsigned long long> dup_tab;  // hash table, only for ids past the replica's boid count
+    DevBuf<uint32_t> id_bits;            // a bit per record: the ids below it that were seen
+    DevBuf<unsigned long long> facts;    // launch_load_facts' results
     // Several replicas: block tables of the force and segment-rebin kernels
     // ({replica, first boid} / {replica, first segment}), no block spanning
     // two replicas; rebuilt with the replica table.
@@ -154,7 +160,7 @@ struct kb_field {
     int32_t dense_mode = KB_DENSE_AUTO;
     bool dense = false;
     DevBuf<unsigned long long> occ_dev;
-    unsigned long long* occ_host = nullptr;  // pinned
+    unsigned long long* occ_host = nullptr;  // pinned: PIN_* words
     cudaEvent_t occ_ev = nullptr;
     bool occ_pending = false;
     uint32_t occ_n = 0;  // boids when the pending measurement was taken
@@ -223,7 +229,7 @@ kb_status upload_rep(kb_field* f);
 // Rebuild a virtual read buffer (after tiled steps).
 kb_status materialize(kb_field* f);
 // The general stable sort of the write list into the read buffer.
-kb_status general_rebuild(kb_field* f, bool counted);
+kb_status general_rebuild(kb_field* f);
 // Field::lazy_update (field_2d.rs:905-921).
 kb_status field_lazy_update(kb_field* f);
 // nsteps steps on the separate kernels (fast: the stencil-gather rebin).
@@ -248,8 +254,9 @@ kb_status autotune_force_block(kb_field* f, uint64_t first_step, uint32_t steps,
                                const int32_t* cand, int32_t ncand, int32_t* best_out,
                                float* best_ms_out, kb_status (*run)(void*, uint64_t, uint32_t),
                                void* ctx);
-// Whether every replica's ids are distinct (checked on the device) / set it.
-kb_status check_unique_ids(kb_field* f);
+// After a general rebuild: the stored count, a plain field's density and whether
+// every replica's ids are distinct (one read back) / set the last.
+kb_status load_facts(kb_field* f, uint32_t most);
 void set_ids_unique(kb_field* f, bool u);
 // Reset the control words of the bounded-wait protocols (after a timeout).
 kb_status reset_wait_state(kb_field* f);

@@ -232,7 +232,36 @@ cudaError_t launch_pack_locations(const Rep& rep, const float2* xy, const float2
 cudaError_t launch_pack_states(const Rep& rep, const float4* st, uint32_t n, float4* out_st,
                                uint32_t* out_key, uint8_t* out_dead, uint32_t* bad, cudaStream_t s);
 
-// General stable counting sort of the write list by key (insertion order
+// The general rebuild: counts (hist zero before; arrival[i] = entry i's arrival
+// number, the bags' first RANK_SLOTS arrivals into slots unless nullptr), and
+// after the offsets scan every live entry to its place in list order.  order:
+// n words of scratch.
+struct PlaceArgs {
+    const uint32_t* key;
+    const uint8_t* dead;
+    const float4* st;
+    const uint32_t* ids;
+    uint32_t n;
+    const uint32_t* arrival;
+    const uint32_t* start;
+    uint32_t ncells;
+    const uint32_t* slots;
+    uint32_t* order;
+    float4* s_st;
+    uint32_t* s_ids;
+};
+cudaError_t launch_count_list(const uint32_t* key, const uint8_t* dead, uint32_t n, uint32_t* hist,
+                              uint32_t* slots, uint32_t ncells, uint32_t* arrival, cudaStream_t s);
+cudaError_t launch_place_list(const PlaceArgs& a, cudaStream_t s);
+// res[0..2] = {sum of squared bag occupancies over ncells bags, id flags (1 a
+// repeat among the ids below their replica's boid count, 2 an id that is not
+// below it), objects stored}; bits: one bit per record (cap of them), cleared
+// with res by the caller.  nboids0: the boid count of a single replica.
+cudaError_t launch_load_facts(const Rep* reps, int32_t nrep, uint32_t nboids0, const uint32_t* ids,
+                              const uint32_t* start, uint32_t ncells, const uint32_t* total, uint32_t cap,
+                              uint32_t* bits, unsigned long long* res, cudaStream_t s);
+
+// Stable counting sort of the write list by key (insertion order
 // kept inside each bag): histogram, scatter, per-bag canonicalisation.
 cudaError_t launch_hist_list(const uint32_t* key, const uint8_t* dead, uint32_t n, uint32_t* hist,
                              cudaStream_t s);
