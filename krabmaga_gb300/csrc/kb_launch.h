@@ -122,11 +122,10 @@ cudaError_t launch_flock_wide(const ForceArgs& a, bool strict, int qmode, cudaSt
 // over rep.ncells bags) into its shared memory, nsteps steps run there, and
 // the final read buffer, offsets and step counter (*step += nsteps) are
 // written back.
-constexpr int SMALL_THREADS = 1024;
 constexpr uint32_t SMALL_CTAS = 8;  // a portable cluster size
-// Measured on GB300 (uniform flocks, 400-step calls): 4.8 / 7.0 / 9.3 / 13.9 us
-// per step at 16 / 1000 / 2048 / 4096 boids, against 13.5 / 14.2 / 14.7 /
-// 15.4 us for the separate kernels; the bound is the shared memory.
+// Measured on GB300 (uniform flocks, 400-step calls): 4.5 / 4.0 / 4.9 / 7.6 us
+// per step at 16 / 1000 / 2048 / 4000 boids, against 8.0 to 8.3 us for the
+// separate kernels; the bound is the shared memory.
 constexpr uint32_t SMALL_MAX_BOIDS = 4096;
 constexpr uint32_t SMALL_MAX_CELLS = 4096;
 struct SmallArgs {

@@ -4,31 +4,37 @@
 // 1,000-boid Flockers case, the reference's own test fields) is launch-bound
 // on the separate-kernel path: four launches per step for a few microseconds
 // of work.  Here a cluster of SMALL_CTAS blocks runs every step of the call
-// in one launch.  Each block holds a full copy of the read buffer and its
-// bag offsets in shared memory and owns one contiguous chunk of the boids:
-//   1. agent pass: Bird::step for the chunk's boids against the local copy
-//      (the same candidate order, accumulator and finish as k_flock_force);
-//      next states and ids go to a local write list, and each bag key is
-//      written into every block's copy of the list of keys (distributed
-//      shared memory);
+// in one launch.  Each block holds the read buffer it needs and all bag offsets
+// in shared memory and owns one contiguous chunk of the boids:
+//   1. agent pass: half of the threads walk the candidates of the chunk's boids
+//      (the same candidate order, accumulator and finish as k_flock_force), the
+//      other half draws their jitter meanwhile; next states and ids go to a
+//      local write list, and the bag keys, eight to a 16-byte store, into every
+//      block's list of keys (distributed shared memory);
 //   -- cluster barrier --
-//   2. lazy_update: every block counts all keys in its own shared memory,
-//      scans the counts into the next bag offsets, and places its own chunk:
-//      position = offset of the bag + arrivals from lower-ranked blocks
-//      (earlier in list order) + rank inside the chunk (one warp walks the
-//      chunk in list order, __match_any_sync ranks equal keys, a per-bag
-//      cursor carries the rank), which is the reference's insertion order
-//      inside a bag; each record is written into every block's copy of the
-//      next read buffer;
+//   2. lazy_update: every block counts all keys in its own shared memory and
+//      scans the counts into the next bag offsets; a boid's place is its bag's
+//      offset, plus the arrivals from lower-ranked blocks (earlier in list
+//      order), plus those of earlier warps of its chunk (one byte per warp and
+//      bag), plus its rank among its warp's equal keys (__match_any_sync): the
+//      reference's insertion order inside a bag.  Each record goes to the blocks
+//      whose next chunk can see its column (to all where queries wrap);
 //   -- cluster barrier --
-// and block 0 writes the final read buffer, offsets and step counter back.
-// No bound on how far a boid moves is needed.
+// and every block writes its chunk of the final read buffer back.  No bound on
+// how far a boid moves is needed.
+//
+// Bound by latency: a step is one pass over some two thousand instructions
+// between barriers, by few warps.  us per step at 300 / 1000 / 2048 / 4000 boids,
+// fast: 3.6 / 4.0 / 4.9 / 7.6, with one warp ranking the chunk in turn, every
+// record sent to all blocks and two candidates at a time without the packed
+// walk 6.5 / 7.1 / 9.3 / 13.8; strict at 1000: 4.8 against 8.6.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "kb_common.h"
 #include "kb_device.cuh"
 #include "kb_launch.h"
+#include "kb_walk.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -53,9 +59,8 @@ __device__ __forceinline__ void take_small(const Rep& R, const uint32_t* ids, ui
 // corner rule (check_circle) for QMODE 1.  Self is the slot my_slot when ids
 // are unique, else every candidate with the boid's id.  The relaxed query of
 // a clamped one-bag ring (the common case) walks its three column runs as one
-// flat list, two candidates per iteration, so the loads and reciprocals of
-// the next candidate overlap the sums of the current one (the sums are still
-// taken in list order: the same bits).
+// flat list, four candidates per iteration, so that their loads and reciprocals
+// overlap (the sums are still taken in list order: the same bits).
 template <bool STRICT, int QMODE>
 __device__ __forceinline__ void gather_small(const Rep& R, const float4* st, const uint32_t* ids,
                                              const uint32_t* start, float4 me, uint32_t my_id,
@@ -74,21 +79,35 @@ __device__ __forceinline__ void gather_small(const Rep& R, const float4* st, con
                 e[k] = start[colbase + (uint32_t)Mj + 1u];
             }
         }
-        const uint32_t P1 = e[0] - s[0], P2 = P1 + (e[1] - s[1]), T = P2 + (e[2] - s[2]);
-        const uint32_t d1 = s[1] - P1, d2 = s[2] - P2;  // position = f + d (mod 2^32)
-        acc.vec += T;
-        uint32_t f = 0;
-        for (; f + 1u < T; f += 2u) {
-            const uint32_t g = f + 1u;
-            const uint32_t p0 = f < P1 ? s[0] + f : (f < P2 ? f + d1 : f + d2);
-            const uint32_t p1 = g < P1 ? s[0] + g : (g < P2 ? g + d1 : g + d2);
-            const float4 o0 = st[p0], o1 = st[p1];
-            take_small(R, ids, p0, o0, me, my_id, my_slot, acc);
-            take_small(R, ids, p1, o1, me, my_id, my_slot, acc);
+        if (R.nowrap && my_slot != 0xFFFFFFFFu) {
+            const Runs r = {{s[0], s[1], s[2]}, {e[0], e[1], e[2]}};
+            pair_t<STRICT> mxy;
+            pack2(mxy, me.x, me.y);
+            Sums<STRICT> sums;
+            walk_flat<STRICT, 4, false>(st, mxy, my_slot, r, sums);
+            bool self_in = false;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) self_in |= my_slot - s[k] < e[k] - s[k];
+            sums.count = sums.vec - (self_in ? 1u : 0u);
+            acc = sums.result();
+            return;
         }
-        if (f < T) {
-            const uint32_t p0 = f < P1 ? s[0] + f : (f < P2 ? f + d1 : f + d2);
-            take_small(R, ids, p0, st[p0], me, my_id, my_slot, acc);
+#pragma unroll 1
+        for (int k = 0; k < 3; ++k) {
+            const uint32_t ks = k == 0 ? s[0] : (k == 1 ? s[1] : s[2]), ke = k == 0 ? e[0] : (k == 1 ? e[1] : e[2]);
+            acc.vec += ke - ks;
+            for (uint32_t q = ks; q < ke; ++q) take_small(R, ids, q, st[q], me, my_id, my_slot, acc);
+        }
+        return;
+    }
+    if (QMODE == 0 && R.toroidal && !R.cell_wrap) {  // wider rings: a run per column
+        if (mj > Mj) return;
+        for (int ci = mi; ci <= Mi; ++ci) {
+            const uint32_t colbase = (uint32_t)ci * (uint32_t)R.dh;
+            const uint32_t e = start[colbase + (uint32_t)Mj + 1u];
+            const uint32_t s = start[colbase + (uint32_t)mj];
+            if (s < e) acc.vec += e - s;
+            for (uint32_t k = s; k < e; ++k) take_small(R, ids, k, st[k], me, my_id, my_slot, acc);
         }
         return;
     }
@@ -118,20 +137,20 @@ __device__ __forceinline__ void gather_small(const Rep& R, const float4* st, con
     }
 }
 
-// Exclusive scan of in[0..n) into out[0..n] (out[n] = total) by one block of
-// SMALL_THREADS threads, n <= SMALL_THREADS * SMALL_SCAN_ITEMS; in may be out.
-constexpr int SMALL_SCAN_ITEMS = (int)SMALL_MAX_CELLS / SMALL_THREADS;
-static_assert(SMALL_SCAN_ITEMS * SMALL_THREADS == (int)SMALL_MAX_CELLS, "scan tiling");
-__device__ __forceinline__ void block_scan_small(const uint32_t* in, uint32_t* out, uint32_t n,
-                                                 uint32_t* warp_sums) {
-    const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5;
-    constexpr uint32_t NW = SMALL_THREADS / 32;
-    const uint32_t b = t * SMALL_SCAN_ITEMS;
-    uint32_t v[SMALL_SCAN_ITEMS], sum = 0;
+// Exclusive scan of v[0..n) in place, v[n] = total, by one block of T threads
+// (n <= SMALL_MAX_CELLS; v has room for whole vectors of 4).
+template <int T>
+__device__ __forceinline__ void block_scan_small(uint32_t* v, uint32_t n, uint32_t* warp_sums) {
+    constexpr int ITEMS = (int)SMALL_MAX_CELLS / T, NW = T / 32;
+    static_assert(ITEMS % 4 == 0 && NW <= 32, "scan tiling");
+    const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5, b = t * ITEMS;
+    uint4 q[ITEMS / 4];
+    uint32_t sum = 0;
 #pragma unroll
-    for (int j = 0; j < SMALL_SCAN_ITEMS; ++j) {
-        v[j] = b + j < n ? in[b + j] : 0u;
-        sum += v[j];
+    for (int j = 0; j < ITEMS / 4; ++j) {
+        q[j] = make_uint4(0u, 0u, 0u, 0u);
+        if (b + 4 * j < n) q[j] = *reinterpret_cast<const uint4*>(v + b + 4 * j);
+        sum += q[j].x + q[j].y + q[j].z + q[j].w;
     }
     uint32_t incl = sum;
 #pragma unroll
@@ -141,155 +160,247 @@ __device__ __forceinline__ void block_scan_small(const uint32_t* in, uint32_t* o
     }
     if (lane == 31u) warp_sums[w] = incl;
     __syncthreads();
-    if (w == 0) {
-        const uint32_t x = lane < NW ? warp_sums[lane] : 0u;
-        uint32_t xi = x;
+    // every warp scans the warp sums itself
+    const uint32_t x = lane < (uint32_t)NW ? warp_sums[lane] : 0u;
+    uint32_t xi = x;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(SMALL_FULL, xi, d);
-            if (lane >= (uint32_t)d) xi += y;
-        }
-        if (lane < NW) warp_sums[lane] = xi - x;  // exclusive prefix of each warp
-        if (lane == 31u) warp_sums[32] = xi;      // total
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(SMALL_FULL, xi, d);
+        if (lane >= (uint32_t)d) xi += y;
     }
-    __syncthreads();
-    uint32_t run = warp_sums[w] + incl - sum;
+    uint32_t run = __shfl_sync(SMALL_FULL, xi - x, w) + incl - sum;
 #pragma unroll
-    for (int j = 0; j < SMALL_SCAN_ITEMS; ++j) {
-        if (b + j < n) out[b + j] = run;
-        run += v[j];
+    for (int j = 0; j < ITEMS / 4; ++j) {
+        uint4 o;
+        o.x = run;
+        o.y = o.x + q[j].x;
+        o.z = o.y + q[j].y;
+        o.w = o.z + q[j].z;
+        run = o.w + q[j].w;
+        if (b + 4 * j < n) *reinterpret_cast<uint4*>(v + b + 4 * j) = o;
     }
-    if (t == 0) out[n] = warp_sums[32];
+    // the total stands behind the last count (its vector may reach past n)
+    const uint32_t total = __shfl_sync(SMALL_FULL, xi, 31);
     __syncthreads();
+    if (t == 0) v[n] = total;
 }
+
+// Boids per block: the chunk, a multiple of 8 (keys travel eight at a time).
+__host__ __device__ inline uint32_t small_chunk(uint32_t n) {
+    return ((n + SMALL_CTAS - 1) / SMALL_CTAS + 7u) / 8u * 8u;
+}
+// Words of warp counters per bag: one byte per warp of the chunk.
+__host__ __device__ inline uint32_t small_words(uint32_t chunk) { return ((chunk + 31u) / 32u + 3u) / 4u; }
 
 // Shared-memory layout (byte offsets), the same in every block of the cluster.
 struct SmallLayout {
-    uint32_t rd_st, wr_st, rd_id, wr_id, wr_key, keys, start, nstart, cnt, cur, bytes;
+    uint32_t rd_st, wr_st, jit, rd_id, wr_id, wr_key, keys, start, nstart, cur, warps, bytes;
 };
 __host__ __device__ inline SmallLayout small_layout(uint32_t n, uint32_t ncells, uint32_t chunk) {
     SmallLayout L{};
     uint32_t o = 0;
+    const uint32_t cells = (ncells + 8u) / 8u * 8u;  // room for one more word and whole vectors
     L.rd_st = o;  o += n * 16u;
     L.wr_st = o;  o += chunk * 16u;
+    L.keys = o;   o += SMALL_CTAS * chunk * 2u;
+    L.jit = o;    o += chunk * 8u;
+    L.start = o;  o += cells * 4u;
+    L.nstart = o; o += cells * 4u;
+    L.warps = o;  o += cells * 4u * small_words(chunk);
+    L.cur = o;    o += cells * 2u;
     L.rd_id = o;  o += n * 4u;
     L.wr_id = o;  o += chunk * 4u;
     L.wr_key = o; o += chunk * 4u;
-    L.keys = o;   o += n * 4u;
-    L.start = o;  o += (ncells + 1u) * 4u;
-    L.nstart = o; o += (ncells + 1u) * 4u;
-    L.cnt = o;    o += ncells * 4u;
-    L.cur = o;    o += ncells * 4u;
     L.bytes = o;
     return L;
 }
 
-template <bool STRICT, int QMODE>
-__global__ void __launch_bounds__(SMALL_THREADS, 1) k_small_steps(SmallArgs a) {
+constexpr uint32_t SMALL_OUTSIDE = 0xFFFFu;  // a key outside the matrix (its boid goes to bag 0)
+constexpr uint32_t SMALL_NONE = 0xFFFEu;     // no boid
+
+// T: threads per block, at least twice the chunk.
+// Shared memory of the cluster's blocks by 32-bit addresses.
+__device__ __forceinline__ uint32_t remote_address(const void* local, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;"
+        : "=r"(r)
+        : "r"((uint32_t)__cvta_generic_to_shared(local)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void store_remote(uint32_t at, uint4 v) {
+    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void store_remote(uint32_t at, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at), "r"(v) : "memory");
+}
+
+template <bool STRICT, int QMODE, int T>
+__global__ void __launch_bounds__(T, 1) k_small_steps(SmallArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     cg::cluster_group cl = cg::this_cluster();
     const Rep& R = a.rep;
     const uint32_t n = a.n, C = R.ncells;
     const uint32_t rank = cl.block_rank();
-    const uint32_t chunk = (n + SMALL_CTAS - 1) / SMALL_CTAS;
-    const uint32_t lo = min(n, rank * chunk), hi = min(n, lo + chunk);
+    const uint32_t chunk = small_chunk(n), words = small_words(chunk);
+    const uint32_t lo = min(n, rank * chunk), m = min(n, lo + chunk) - lo;
     const SmallLayout Lo = small_layout(n, C, chunk);
     float4* rd_st = reinterpret_cast<float4*>(smem + Lo.rd_st);
     uint32_t* rd_id = reinterpret_cast<uint32_t*>(smem + Lo.rd_id);
     uint32_t* start = reinterpret_cast<uint32_t*>(smem + Lo.start);
-    uint32_t* nstart = reinterpret_cast<uint32_t*>(smem + Lo.nstart);
-    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem + Lo.cnt);  // arrivals per bag
-    uint32_t* cur = reinterpret_cast<uint32_t*>(smem + Lo.cur);  // lower-ranked arrivals, cursors
-    uint32_t* keys = reinterpret_cast<uint32_t*>(smem + Lo.keys);  // every boid's next bag
+    uint32_t* nstart = reinterpret_cast<uint32_t*>(smem + Lo.nstart);  // arrivals per bag, then offsets
+    uint32_t* cur = reinterpret_cast<uint32_t*>(smem + Lo.cur);  // arrivals from lower-ranked blocks, 16 bits a bag
+    uint32_t* warps = reinterpret_cast<uint32_t*>(smem + Lo.warps);  // arrivals per warp of the chunk, a byte each
+    uint16_t* keys = reinterpret_cast<uint16_t*>(smem + Lo.keys);  // every boid's next bag
     float4* wr_st = reinterpret_cast<float4*>(smem + Lo.wr_st);
+    float2* jit = reinterpret_cast<float2*>(smem + Lo.jit);
     uint32_t* wr_id = reinterpret_cast<uint32_t*>(smem + Lo.wr_id);
     uint32_t* wr_key = reinterpret_cast<uint32_t*>(smem + Lo.wr_key);
-    __shared__ uint32_t warp_sums[33];
-    __shared__ uint32_t s_err;
-    const uint32_t t = threadIdx.x;
-    for (uint32_t i = t; i < n; i += blockDim.x) {
+    __shared__ uint32_t warp_sums[32];
+    __shared__ uint32_t line[2][SMALL_CTAS];  // columns of each block's next first and last boid
+    __shared__ uint32_t s_err, s_all;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    const uint32_t walkers = (chunk + 31u) / 32u * 32u;  // whole warps
+    for (uint32_t i = t; i < n; i += T) {
         rd_st[i] = a.st[i];
         rd_id[i] = a.ids[i];
     }
-    for (uint32_t c = t; c <= C; c += blockDim.x) start[c] = a.start[c];
-    if (t == 0) s_err = 0u;
+    for (uint32_t c = t; c <= C; c += T) start[c] = a.start[c];
+    for (uint32_t c = t; c < C * words; c += T) warps[c] = 0u;
+    if (t < 2u * SMALL_CTAS) line[t / SMALL_CTAS][t % SMALL_CTAS] = 0u;
+    if (t == 0) {
+        s_err = 0u;
+        // records go to every block where a query can wrap, and from the step
+        // on in which a position fell outside the matrix
+        s_all = R.toroidal && !R.cell_wrap ? 0u : 1u;
+    }
+    // a thread writes to one other block: keys, records and ids of block t % 8
+    static_assert(T % SMALL_CTAS == 0 && SMALL_CTAS == 8, "one target block per thread");
+    const uint32_t key_q = remote_address(keys, t % SMALL_CTAS);
+    const uint32_t st_q = remote_address(rd_st, t % SMALL_CTAS), id_q = remote_address(rd_id, t % SMALL_CTAS);
     unsigned long long step = *a.step;
     // every block of the cluster is running (its shared memory may be written
     // through the cluster) and has its whole copy loaded before any thread
     // reads a neighbour
     cl.sync();
     for (uint32_t s = 0; s < a.nsteps; ++s, ++step) {
-        // 1. agent pass over the own chunk
-        for (uint32_t c = t; c < C; c += blockDim.x) {
-            cnt[c] = 0u;
-            cur[c] = 0u;
+        // 1. agent pass over the own chunk: candidates by the first threads,
+        //    jitter by the last
+        if (t >= walkers) {  // meanwhile: the counters
+            for (uint32_t c = t - walkers; c < C; c += T - walkers) nstart[c] = 0u;
+            for (uint32_t c = t - walkers; c < (C + 1u) / 2u; c += T - walkers) cur[c] = 0u;
         }
-        for (uint32_t i = lo + t; i < hi; i += blockDim.x) {
-            const float4 me = rd_st[i];
-            const uint32_t my_id = rd_id[i];
-            Acc<STRICT> acc;
-            gather_small<STRICT, QMODE>(R, rd_st, rd_id, start, me, my_id,
-                                        a.self_by_slot ? i : 0xFFFFFFFFu, acc);
-            const float4 nx = finish_bird<STRICT>(R, me, my_id, step, acc);
-            int64_t idx = bag_index(R, disc(nx.x, R), disc(nx.y, R));
-            uint32_t flags = 0;
-            if (idx < 0) {
-                flags |= ERR_KEY_RANGE;
-                idx = 0;
+        Acc<STRICT> acc;
+        float4 me = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < m) {
+            me = rd_st[lo + t];
+            gather_small<STRICT, QMODE>(R, rd_st, rd_id, start, me, rd_id[lo + t],
+                                        a.self_by_slot ? lo + t : 0xFFFFFFFFu, acc);
+        } else if (t >= T / 2 && t - T / 2 < m) {
+            jit[t - T / 2] = bird_jitter<STRICT>(R, rd_id[lo + t - T / 2], step);
+        }
+        __syncthreads();
+        if (t < walkers) {
+            uint32_t key = SMALL_NONE;
+            if (t < m) {
+                const float4 nx = finish_bird_with<STRICT>(R, me, acc, [&] { return jit[t]; });
+                const int64_t idx = bag_index(R, disc(nx.x, R), disc(nx.y, R));
+                uint32_t flags = 0;
+                if (idx < 0) flags |= ERR_KEY_RANGE;
+                if (!isfinite(nx.x) || !isfinite(nx.y)) flags |= ERR_NONFINITE;
+                if (flags) atomicOr(&s_err, flags);
+                key = idx < 0 ? SMALL_OUTSIDE : (uint32_t)idx;
+                wr_st[t] = nx;
+                wr_id[t] = rd_id[lo + t];
+                wr_key[t] = idx < 0 ? 0u : (uint32_t)idx;
             }
-            if (!isfinite(nx.x) || !isfinite(nx.y)) flags |= ERR_NONFINITE;
-            if (flags) atomicOr(&s_err, flags);
-            wr_st[i - lo] = nx;
-            wr_id[i - lo] = my_id;
-            wr_key[i - lo] = (uint32_t)idx;
+            // eight keys a store, lane q of each eight to block q
+            uint32_t w[4];
 #pragma unroll
-            for (uint32_t q = 0; q < SMALL_CTAS; ++q) *cl.map_shared_rank(keys + i, q) = (uint32_t)idx;
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t k0 = __shfl_sync(SMALL_FULL, key, (lane & 24u) + 2 * k);
+                const uint32_t k1 = __shfl_sync(SMALL_FULL, key, (lane & 24u) + 2 * k + 1);
+                w[k] = k0 | (k1 << 16);
+            }
+            const uint32_t at = t & ~7u;
+            if (at < chunk) store_remote(key_q + (rank * chunk + at) * 2u, make_uint4(w[0], w[1], w[2], w[3]));
         }
         cl.sync();  // every copy of the keys is complete; no block reads rd_* any more
-        // 2. next offsets (all arrivals) and this chunk's cursors (arrivals
-        //    from lower-ranked blocks, earlier in the list, come first in a bag)
-        for (uint32_t i = t; i < n; i += blockDim.x) {
-            atomicAdd(&cnt[keys[i]], 1u);
-            if (i < lo) atomicAdd(&cur[keys[i]], 1u);
+        // 2. arrivals per bag, and per bag those of lower-ranked blocks (earlier
+        //    in the list)
+        for (uint32_t i = t; i < SMALL_CTAS * chunk; i += T) {
+            uint32_t k = keys[i];
+            if (k == SMALL_NONE) continue;
+            if (k == SMALL_OUTSIDE) {
+                k = 0u;
+                s_all = 1u;
+            }
+            atomicAdd(&nstart[k], 1u);
+            if (i < lo) atomicAdd(&cur[k >> 1], 1u << (16u * (k & 1u)));
+        }
+        // equal keys of a warp of the chunk
+        uint32_t my_key = 0, r = 0;
+        if (t < walkers) {
+            const bool valid = t < m;
+            my_key = valid ? wr_key[t] : 0xFFFFFFFFu;
+            const uint32_t peers = __match_any_sync(SMALL_FULL, my_key);
+            r = __popc(peers & ((1u << lane) - 1u));
+            if (valid && r == 0u)
+                atomicAdd(&warps[my_key * words + (warp >> 2)], (uint32_t)__popc(peers) << (8u * (warp & 3u)));
         }
         __syncthreads();
-        block_scan_small(cnt, nstart, C, warp_sums);
-        for (uint32_t c = t; c < C; c += blockDim.x) cur[c] += nstart[c];
+        block_scan_small<T>(nstart, C, warp_sums);
         __syncthreads();
-        if (t < 32u) {
-            const uint32_t lt = (1u << t) - 1u;
-            for (uint32_t base = 0; base < hi - lo; base += 32u) {
-                const uint32_t j = base + t;
-                const bool valid = j < hi - lo;
-                const uint32_t k = valid ? wr_key[j] : 0xFFFFFFFFu;
-                const uint32_t peers = __match_any_sync(SMALL_FULL, k);
-                const uint32_t r = __popc(peers & lt);
-                const uint32_t pos = valid ? cur[k] + r : 0u;
-                __syncwarp();
-                if (valid) {
-                    if (r + 1u == (uint32_t)__popc(peers)) cur[k] = pos + 1u;
-                    wr_key[j] = pos;  // the key becomes the destination slot
+        if (t >= T / 2) {  // the columns of every chunk's first and last boid
+            for (uint32_t x = t - T / 2; x < (uint32_t)R.dw; x += T / 2) {
+                const uint32_t from = nstart[x * (uint32_t)R.dh], to = nstart[(x + 1u) * (uint32_t)R.dh];
+#pragma unroll
+                for (uint32_t q = 0; q < SMALL_CTAS; ++q) {
+                    const uint32_t first = q * chunk, last = min(n, first + chunk) - 1u;
+                    if (first < n && first - from < to - from) line[0][q] = x;
+                    if (first < n && last - from < to - from) line[1][q] = x;
                 }
-                __syncwarp();
             }
         }
-        __syncthreads();
-        // every block's copy of the next read buffer gets this chunk
-        for (uint32_t x = t; x < (hi - lo) * SMALL_CTAS; x += blockDim.x) {
-            const uint32_t j = x / SMALL_CTAS, q = x % SMALL_CTAS;
-            const uint32_t pos = wr_key[j];
-            *cl.map_shared_rank(rd_st + pos, q) = wr_st[j];
-            *cl.map_shared_rank(rd_id + pos, q) = wr_id[j];
+        if (t < m) {
+            uint32_t before = r;
+            for (uint32_t q = 0; q < words; ++q) {
+                uint32_t v = warps[my_key * words + q];
+                if (q == (warp >> 2)) v &= (1u << (8u * (warp & 3u))) - 1u;
+                else if (q > (warp >> 2)) v = 0u;
+                before += (uint32_t)__dp4a(v, 0x01010101u, 0u);
+            }
+            const uint32_t lower = (cur[my_key >> 1] >> (16u * (my_key & 1u))) & 0xFFFFu;
+            wr_key[t] = nstart[my_key] + lower + before;  // the key becomes the destination slot
         }
-        for (uint32_t c = t; c <= C; c += blockDim.x) start[c] = nstart[c];
+        __syncthreads();
+        if (t < m)
+            for (uint32_t q = 0; q < words; ++q) warps[my_key * words + q] = 0u;
+        // the blocks whose next chunk can see a record get it
+        const uint32_t q = t % SMALL_CTAS;
+        uint32_t from = 0u, to = n;
+        if (s_all == 0u) {
+            const uint32_t dd = (uint32_t)max(R.dd, 0), x0 = line[0][q];
+            from = nstart[(x0 > dd ? x0 - dd : 0u) * (uint32_t)R.dh];
+            to = q * chunk < n ? nstart[(min(line[1][q] + dd, (uint32_t)R.dw - 1u) + 1u) * (uint32_t)R.dh] : from;
+        }
+        for (uint32_t j = t / SMALL_CTAS; j < m; j += T / SMALL_CTAS) {
+            const uint32_t pos = wr_key[j];
+            if (pos - from < to - from) {
+                store_remote(st_q + pos * 16u, reinterpret_cast<const uint4*>(wr_st)[j]);
+                store_remote(id_q + pos * 4u, wr_id[j]);
+            }
+        }
+        uint32_t* const o = start;
+        start = nstart;
+        nstart = o;
         cl.sync();  // every copy of the next read buffer is complete; counters are free
     }
+    if (t < m) {
+        a.st[lo + t] = rd_st[lo + t];
+        a.ids[lo + t] = rd_id[lo + t];
+    }
     if (rank == 0) {
-        for (uint32_t i = t; i < n; i += blockDim.x) {
-            a.st[i] = rd_st[i];
-            a.ids[i] = rd_id[i];
-        }
-        for (uint32_t c = t; c <= C; c += blockDim.x) a.start[c] = start[c];
+        for (uint32_t c = t; c <= C; c += T) a.start[c] = start[c];
         if (t == 0) *a.step = step;
     }
     __syncthreads();
@@ -298,17 +409,14 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small_steps(SmallArgs a) {
 
 }  // namespace
 
-size_t small_smem_bytes(uint32_t n, uint32_t ncells) {
-    return small_layout(n, ncells, (n + SMALL_CTAS - 1) / SMALL_CTAS).bytes;
-}
+size_t small_smem_bytes(uint32_t n, uint32_t ncells) { return small_layout(n, ncells, small_chunk(n)).bytes; }
 
-cudaError_t launch_small_steps(const SmallArgs& a, bool strict, int qmode, cudaStream_t s) {
-    if (a.nsteps == 0) return cudaSuccess;
-    if (a.n == 0 || a.n > SMALL_MAX_BOIDS || a.rep.ncells > SMALL_MAX_CELLS || a.rep.cell_off != 0)
-        return cudaErrorInvalidValue;
-    const size_t bytes = small_smem_bytes(a.n, a.rep.ncells);
-    void (*k)(SmallArgs) = strict ? (qmode == 0 ? k_small_steps<true, 0> : k_small_steps<true, 1>)
-                                  : (qmode == 0 ? k_small_steps<false, 0> : k_small_steps<false, 1>);
+namespace {
+
+template <int T>
+cudaError_t launch_small(const SmallArgs& a, bool strict, int qmode, cudaStream_t s) {
+    void (*k)(SmallArgs) = strict ? (qmode == 0 ? k_small_steps<true, 0, T> : k_small_steps<true, 1, T>)
+                                  : (qmode == 0 ? k_small_steps<false, 0, T> : k_small_steps<false, 1, T>);
     // the largest layout once per kernel (and device), not per launch
     static thread_local int opted[4] = {-1, -1, -1, -1};
     const int ki = (strict ? 2 : 0) + (qmode == 0 ? 0 : 1);
@@ -323,8 +431,8 @@ cudaError_t launch_small_steps(const SmallArgs& a, bool strict, int qmode, cudaS
     }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(SMALL_CTAS, 1, 1);
-    cfg.blockDim = dim3(SMALL_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = bytes;
+    cfg.blockDim = dim3(T, 1, 1);
+    cfg.dynamicSmemBytes = small_smem_bytes(a.n, a.rep.ncells);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -334,6 +442,17 @@ cudaError_t launch_small_steps(const SmallArgs& a, bool strict, int qmode, cudaS
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k, a);
+}
+
+}  // namespace
+
+cudaError_t launch_small_steps(const SmallArgs& a, bool strict, int qmode, cudaStream_t s) {
+    if (a.nsteps == 0) return cudaSuccess;
+    if (a.n == 0 || a.n > SMALL_MAX_BOIDS || a.rep.ncells > SMALL_MAX_CELLS || a.rep.cell_off != 0)
+        return cudaErrorInvalidValue;
+    // two threads per boid of a chunk: fewer warps at every barrier for small flocks
+    return small_chunk(a.n) <= 256u ? launch_small<512>(a, strict, qmode, s)
+                                    : launch_small<1024>(a, strict, qmode, s);
 }
 
 }  // namespace kb
