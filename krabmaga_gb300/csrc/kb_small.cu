@@ -138,7 +138,7 @@ __device__ __forceinline__ void gather_small(const Rep& R, const float4* st, con
 }
 
 // Exclusive scan of v[0..n) in place, v[n] = total, by one block of T threads
-// (n <= SMALL_MAX_CELLS; v has room for whole vectors of 4).
+// (n <= SMALL_MAX_CELLS; v has room for whole vectors of 4, zero past n).
 template <int T>
 __device__ __forceinline__ void block_scan_small(uint32_t* v, uint32_t n, uint32_t* warp_sums) {
     constexpr int ITEMS = (int)SMALL_MAX_CELLS / T, NW = T / 32;
@@ -286,7 +286,8 @@ __global__ void __launch_bounds__(T, 1) k_small_steps(SmallArgs a) {
         // 1. agent pass over the own chunk: candidates by the first threads,
         //    jitter by the last
         if (t >= walkers) {  // meanwhile: the counters
-            for (uint32_t c = t - walkers; c < C; c += T - walkers) nstart[c] = 0u;
+            // (to the end of the last whole vector, which the scan adds up)
+            for (uint32_t c = t - walkers; c < (C + 4u) / 4u * 4u; c += T - walkers) nstart[c] = 0u;
             for (uint32_t c = t - walkers; c < (C + 1u) / 2u; c += T - walkers) cur[c] = 0u;
         }
         Acc<STRICT> acc;

@@ -158,3 +158,28 @@ def test_small_path_random_fields_equal_separate_kernels(gpu):
         (ia, sa), (ib, sb) = out
         assert np.array_equal(ia, ib) and same_bits(sa, sb), (case, n, side, d, tor, wrap, kind)
     assert ran >= 12
+
+
+@pytest.mark.parametrize("lines", [9, 10, 11, 12, 64])
+def test_small_path_bag_counts_past_whole_vectors(gpu, lines):
+    # (lines)^2 bags: every remainder of four; the offsets end in the boid count
+    d = 5.0
+    side, n = d * (lines - 1), 700
+    ids, xy, dxy = kg.gen_uniform(n, side, side, lines, 1.0)
+    p = kg.FlockParams(seed=lines, arith=kg.KB_ARITH_STRICT, neighbor_radius=7.5)
+    for _ in range(3):  # whatever an earlier launch left in shared memory
+        f = kg.Field2D(side, side, d, True)
+        f.set_locations(ids, xy, dxy)
+        f.lazy_update()
+        assert f.step_path() == kg.KB_PATH_SMALL and f.dw == lines
+        f.flock_step(p, 0, 5)
+        f.flock_step(p, 5, 1)  # a single step on the offsets the first call left
+        gi, gs = f.get_state()
+        assert f.moments()[0] == n
+        f.close()
+        o = oracle.OracleField(side, side, d, True)
+        o.set_many(ids, xy, dxy)
+        o.lazy_update()
+        o.flock_run(oracle.params_from(p), 0, 6)
+        oi, os_, _ = o.iter(1)
+        assert np.array_equal(gi, oi) and np.array_equal(gs.view(np.uint32), os_.view(np.uint32))
