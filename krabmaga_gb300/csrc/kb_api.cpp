@@ -2220,10 +2220,11 @@ static kb_status flock_step_impl(kb_field* f, const kb_flock_params* p, uint64_t
     }
     if (done < nsteps && fused_eligible(f, p)) return tiled_steps(f, p, nsteps - done);
     if (f->virt && (st = materialize(f))) return st;
-    if (small_eligible(f) && nsteps - done >= 2) {
-        // a small field: whole steps in one cluster, up to 1000 per launch
-        // (a single step is quicker on the separate kernels: the cluster's
-        // launch, load and write-back cost more than it saves there)
+    if (small_eligible(f) && (nsteps - done >= 2 || !f->ktime)) {
+        // a small field: whole steps in one cluster, up to 1000 per launch.  A
+        // single step too (a frame of 1,000 boids, step and state read: 47 us,
+        // 50 to 54 with the separate kernels' four launches), unless its kernels
+        // are being timed.
         while (done < nsteps) {
             const uint32_t k = std::min<uint32_t>(1000u, nsteps - done);
             SmallArgs a{};
