@@ -551,6 +551,9 @@ kb_status fast_rebuild(kb_field* f, bool bump_step, bool stencil) {
 bool ring_ok(const kb_field* f, bool* wide) {
     *wide = false;
     if (!f->ids_unique || f->rn > (1u << 26)) return false;
+    // objects set apart from their own positions: the exact query's distances
+    // can wrap although no ring does
+    if (!f->layout_is_positions && f->reps[0].qmode != KB_QUERY_RELAX) return false;
     bool one = true;
     for (const Rep& R : f->reps) {
         if (!R.toroidal || R.cell_wrap || !R.nowrap) return false;

@@ -122,3 +122,35 @@ def test_ring_kernels_equal_the_general_kernel(gpu, kind, arith):
         out.append((gi[rest], gs[rest].view(np.uint32)))
         f.close()
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("d,radius", [(10.0 / 1.5, 10.0), (2.0, 9.0)])
+@pytest.mark.parametrize("kind", [kg.KB_QUERY_RELAX, kg.KB_QUERY_EXACT])
+def test_objects_apart_from_their_positions_match_oracle(gpu, kind, d, radius):
+    # the first step reads bags that objects were set in, from wherever they are
+    side, n = 100.0, 150
+    r = np.random.default_rng(3)
+    pos = r.uniform(0, side * (1 - 1e-6), (n, 2)).astype(np.float32)
+    loc = pos.copy()
+    # anywhere; under the relaxed query near enough that no pair straddles the seam
+    reach = 15.0 if kind == kg.KB_QUERY_RELAX else side
+    loc[::3] = np.clip(loc[::3] + r.uniform(-reach, reach, loc[::3].shape), 0, side * (1 - 1e-6)).astype(np.float32)
+    f, o = kg.Field2D(side, side, d, True), oracle.OracleField(side, side, d, True)
+    f.set_step_options(3)
+    for i in range(n):
+        b = kg.Bird(i, kg.Real2D(float(pos[i, 0]), float(pos[i, 1])), kg.Real2D(0.6, 0.8))
+        f.set_object_location(b, kg.Real2D(float(loc[i, 0]), float(loc[i, 1])))
+        o.set(i, pos[i, 0], pos[i, 1], 0.6, 0.8, loc[i, 0], loc[i, 1])
+    f.lazy_update()
+    o.lazy_update()
+    q = r.uniform(-d, side + d, (400, 2)).astype(np.float32)
+    gc, gi = f.neighbor_lists(kind, radius, q)
+    oc, oi = o.neighbor_lists(kind, radius, q)
+    assert np.array_equal(gc, oc) and np.array_equal(gi, oi)
+    p = kg.FlockParams(seed=5, arith=kg.KB_ARITH_STRICT, query_mode=kind, neighbor_radius=radius)
+    f.flock_step(p, 0, 3)
+    o.flock_run(oracle.params_from(p), 0, 3)
+    oids, ost, _ = o.iter(1)
+    g = f.get_state()
+    assert np.array_equal(g[0], oids) and np.array_equal(g[1].view(np.uint32), ost.view(np.uint32))
+    f.close()
