@@ -142,6 +142,17 @@ void set_rep_params(Rep* R, const kb_flock_params* p) {
     R->seam = (int32_t)std::max(0.0, std::min(lo, (double)R->max_x));
 }
 
+// A point may lie anywhere, also beyond the matrix, where the clamped range does
+// not hold its own bag: its distances are those of the ring only inside.
+void query_ring_args(QueryArgs* a) {
+    const Rep& R = a->rep;
+    const float dist = a->dist;
+    a->thr = sqrt_threshold(dist);
+    const double reach = 2.0 * (double)R.d;
+    a->ring = (R.toroidal && !R.cell_wrap && dist > 0.0f && as_i32(std::floor(dist / R.d)) <= 1 &&
+               reach * 1.01 + 1e-3 < 0.5 * (double)std::min(R.w, R.h)) ? 1 : 0;
+}
+
 bool params_ok(const kb_flock_params* p, std::string* why) {
     const float v[7] = {p->cohesion, p->avoidance, p->consistency, p->randomness,
                         p->momentum, p->jump,      p->neighbor_radius};

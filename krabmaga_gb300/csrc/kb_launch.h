@@ -290,7 +290,13 @@ struct QueryArgs {
     uint32_t* out_ids;
     float4* out_st;
     uint64_t cap;
+    // set by launch_query: the range is clamped and at most one bag around the
+    // point's own, and no distance in it wraps; the largest square within dist
+    int32_t ring;
+    float thr;
 };
+// ring and thr of a query by its geometry and distance.
+void query_ring_args(QueryArgs* a);
 cudaError_t launch_query(const QueryArgs& a, cudaStream_t s);
 
 // Ordered filter of the write list: entries with key == target and not dead,
