@@ -1030,11 +1030,10 @@ __global__ void __launch_bounds__(32 * REBIN_SEG_WARPS, MULTI ? KB_REBIN_MINB_MU
 template <bool MULTI>
 __device__ __noinline__ void place_by_lines(const RebinArgs& a, bool over, uint32_t i) {
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t key = 0, first = 0, cnt = 0, rank = 0;
+    uint32_t key = 0, first = 0, rank = 0;
     if (over) {
         key = __ldcg(a.key + i);
         first = __ldg(a.start_next + key);
-        cnt = min(__ldg(a.start_next + key + 1), a.n) - first;
     }
     uint32_t pending = __ballot_sync(FULL_MASK, over);
     while (pending) {
@@ -1045,13 +1044,14 @@ __device__ __noinline__ void place_by_lines(const RebinArgs& a, bool over, uint3
         const uint32_t local = k - R.cell_off;
         const uint32_t Xu = div_dh(local, R);
         const int X = (int)Xu, Y = (int)(local - Xu * (uint32_t)R.dh);
-        uint32_t total = 0;
-        auto count = [&](uint32_t s, uint32_t e) {
+        // nothing behind the last entry of this key matters
+        const uint32_t last = __reduce_max_sync(FULL_MASK, mine ? i : 0u);
+        auto count = [&](uint32_t s, uint32_t e0) {
+            const uint32_t e = min(e0, last);
 #pragma unroll 2
             for (uint32_t p = s; p < e; p += 32u) {
                 const bool hit = p + lane < e && __ldg(a.key + p + lane) == k;
                 const uint32_t m = __ballot_sync(FULL_MASK, hit);
-                total += __popc(m);
                 // entries p .. i-1 of this batch
                 const uint32_t d = i > p ? i - p : 0u;
                 rank += mine ? __popc(d >= 32u ? m : m & ((1u << d) - 1u)) : 0;
@@ -1085,7 +1085,6 @@ __device__ __noinline__ void place_by_lines(const RebinArgs& a, bool over, uint3
                 }
             }
         }
-        if (mine && total != cnt) atomicOr(a.err, ERR_REBIN_MISS | ERR_MISS_MATERIALIZE);
         pending &= ~__ballot_sync(FULL_MASK, mine);
     }
     if (over && first + rank < a.n) {
@@ -1099,7 +1098,8 @@ __device__ __noinline__ void place_by_lines(const RebinArgs& a, bool over, uint3
 // with one entry per thread, 13.0 with two, 15.3 with four; step 43.8 / 41.9 /
 // 43.6 us).  Fuller bags by warps rather than by each boid alone: 64 replicas
 // whose flocks condense over 500 steps, last 100 steps 105 us each against 113
-// for 64-bag segments (per-boid walks: no gain over segments there).
+// for 64-bag segments (per-boid walks: no gain over segments there); with the
+// ring force kernels 93, and 89 since a key's count stops at its last entry.
 constexpr int RANK_ITEMS = 2;
 constexpr int RANK_THREADS = 256;
 template <bool MULTI>
