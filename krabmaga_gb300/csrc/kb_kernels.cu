@@ -1857,7 +1857,7 @@ cudaError_t launch_flock_force(const ForceArgs& a, bool strict, int qmode, cudaS
     const bool multi = a.nrep > 1;
     if (multi && a.blk == nullptr) return cudaErrorInvalidValue;
     if (a.wide) return launch_flock_wide(a, strict, qmode, s);
-    if (a.ring && (strict || qmode != 0 || !a.dense)) return launch_flock_ring(a, strict, qmode, s);
+    if (a.ring) return launch_flock_ring(a, strict, qmode, s);
     const unsigned g = multi ? a.nblk : grid_for(a.n, KB_FORCE_THREADS);
 #define KB_FORCE(S, Q, MU)                                                                      \
     do {                                                                                        \
