@@ -20,6 +20,8 @@ struct ScanCtl {
 };
 constexpr uint32_t SCAN_TILE = 4096;  // items per CTA (256 threads x 16)
 inline uint32_t scan_tiles(uint32_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE; }
+constexpr uint32_t SCAN_CLUSTER = 8;  // blocks of the one-launch cluster scan
+constexpr uint32_t SCAN_CLUSTER_MAX = SCAN_CLUSTER * 1024u * 4u;  // its bags
 // Items per tile of the two-pass scan (inputs of up to SCAN2_MAX_TILES tiles).
 #ifndef KB_SCAN2_ITEMS
 #define KB_SCAN2_ITEMS 4
