@@ -199,14 +199,21 @@ kb_status grow(kb_field* f, uint32_t need) {
     if (nc > 0xFFFFFFF0ull) nc = 0xFFFFFFF0ull;
     if (need > nc) return fail(KB_ERR_ARG, "object count exceeds 2^32-16");
     const uint32_t c = (uint32_t)nc;
-    DevBuf<float4> rst, wst, tst;
-    DevBuf<uint32_t> rid, wid, wkey, tid, tsrc;
+    DevBuf<float4> recs, rst, wst, tst;
+    DevBuf<uint32_t> words, rid, wid, wkey, tid, tsrc;
     DevBuf<uint8_t> wdead;
+    const size_t part = ((size_t)c + 3u) / 4u * 4u;  // 16-byte parts
     cudaError_t e;
-    if ((e = rst.alloc(c)) || (e = wst.alloc(c)) || (e = tst.alloc(c)) || (e = rid.alloc(c)) ||
-        (e = wid.alloc(c)) || (e = wkey.alloc(c)) || (e = tid.alloc(c)) || (e = tsrc.alloc(c)) ||
-        (e = wdead.alloc(c)))
+    if ((e = recs.alloc(3 * (size_t)c)) || (e = words.alloc(5 * part)) || (e = wdead.alloc(c)))
         return cuda_fail(e, "growing object storage");
+    rst.view(recs.p, c);
+    wst.view(recs.p + c, c);
+    tst.view(recs.p + 2 * (size_t)c, c);
+    rid.view(words.p, c);
+    wid.view(words.p + part, c);
+    wkey.view(words.p + 2 * part, c);
+    tid.view(words.p + 3 * part, c);
+    tsrc.view(words.p + 4 * part, c);
     // no removal marks outside the live write list (they are cleared as consumed)
     KB_CUDA(cudaMemsetAsync(wdead.p, 0, c, f->stream));
     if (f->rn) {
@@ -220,6 +227,7 @@ kb_status grow(kb_field* f, uint32_t need) {
         KB_CUDA(cudaMemcpyAsync(wdead.p, f->wdead.p, f->wn, cudaMemcpyDeviceToDevice, f->stream));
     }
     KB_CUDA(cudaStreamSynchronize(f->stream));
+    f->rec_slab.swap(recs); f->id_slab.swap(words);
     f->rst.swap(rst); f->wst.swap(wst); f->tst.swap(tst);
     f->rid.swap(rid); f->wid.swap(wid); f->wkey.swap(wkey);
     f->tid.swap(tid); f->tsrc.swap(tsrc); f->wdead.swap(wdead);

@@ -35,6 +35,10 @@ struct kb_field {
     unsigned long long dstep_host = 0;  // the device step counter once queued work has run
     bool is_batch = false;
     DevBuf<Rep> d_rep;
+    // the record and the id and key arrays below, one allocation each (declared
+    // before their parts, so freed after them)
+    DevBuf<float4> rec_slab;
+    DevBuf<uint32_t> id_slab;
     // read buffer
     uint32_t cap = 0;
     DevBuf<float4> rst;

@@ -26,6 +26,7 @@ template <typename T>
 struct DevBuf {
     T* p = nullptr;
     size_t n = 0;
+    bool own = true;  // false: a part of another buffer (view)
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
@@ -46,17 +47,26 @@ struct DevBuf {
         n = count;
         return cudaSuccess;
     }
+    // Become `count` elements at q, which another buffer owns.
+    void view(T* q, size_t count) {
+        release();
+        p = q;
+        n = count;
+        own = false;
+    }
     void release() {
-        if (p) {
+        if (p && own) {
             g_dev_frees.fetch_add(1, std::memory_order_relaxed);
             cudaFree(p);
         }
         p = nullptr;
         n = 0;
+        own = true;
     }
     void swap(DevBuf& o) {
         std::swap(p, o.p);
         std::swap(n, o.n);
+        std::swap(own, o.own);
     }
 };
 
