@@ -294,7 +294,7 @@ def run_sweep(args, dev):
         "unit": UNIT, "batched_ms_per_step": best["ms_per_step"], "best_mode": best["mode"],
         "modes": runs,
         "launch": "mode 2: tile step + scan per step, CUDA graphs of 100 steps; mode 0: force + "
-                  "offsets scan (three launches at this bag count) + rebin (64-bag segments) per "
+                  "offsets scan (three launches at this bag count) + ranked rebin per "
                   "step over all replicas, CUDA graphs of 100 steps, programmatic dependent "
                   "launch between the kernels",
         "data": "synthetic (seeded)", "l2": "working set larger than L2 (no flush)",
@@ -559,8 +559,9 @@ def run_ours(args, wl):
     kernels = None
     if kernel_ms is not None and kernel_steps == K:
         fm, sm, rm = (v / K for v in kernel_ms)
-        kernels = {"k_flock_force": {"ms_mean": fm, "impl_bytes": force_bytes,
-                                     "impl_gbs": force_bytes / fm / 1e6}}
+        force_name = "k_flock_dense" if dense and args.arith == "fast" else "k_flock_ring"
+        kernels = {force_name: {"ms_mean": fm, "impl_bytes": force_bytes,
+                                "impl_gbs": force_bytes / fm / 1e6}}
         if sm < 1e-3:  # the offsets scan runs inside the rebin launch
             ob = scan_bytes + rebin_bytes
             kernels["k_offsets_rebin"] = {"ms_mean": sm + rm, "impl_bytes": ob,
@@ -570,7 +571,7 @@ def run_ours(args, wl):
                                  "impl_gbs": scan_bytes / sm / 1e6}
             kernels["k_rebin"] = {"ms_mean": rm, "impl_bytes": rebin_bytes,
                                   "impl_gbs": rebin_bytes / rm / 1e6}
-        kname, kbytes, kms = "k_flock_force", step_bytes, fm
+        kname, kbytes, kms = force_name, step_bytes, fm
     else:  # tiled modes: the whole step is the measured unit
         kname = {2: "k_tile_step + k_scan (two launches per step)",
                  1: "k_fused (whole step, one launch)", 0: "whole step"}[args.mode]

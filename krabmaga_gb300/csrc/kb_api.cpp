@@ -520,6 +520,7 @@ kb_status general_rebuild(kb_field* f) {
     a.order = f->tsrc.p;
     a.s_st = f->rst.p;
     a.s_ids = f->rid.p;
+    a.err = f->err.p;
     KB_CUDA(launch_place_list(a, s));
     f->cur = nxt;
     return KB_OK;

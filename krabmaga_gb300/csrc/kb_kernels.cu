@@ -6,8 +6,9 @@
 //                insertion order; start[ncells+1] u32 bag offsets.
 //   write list   the same records in arbitrary order plus a u32 bag key each
 //                (the write buffer of field_2d.rs:838-846).
-// A flock step is: force pass (read buffer -> write list, key histogram),
-// scan of the histogram, stencil-gather rebin (write list -> read buffer).
+// A flock step is: force pass (read buffer -> write list, key histogram and
+// arrival slots; here, in kb_ring.cu or kb_wide.cu), scan of the histogram,
+// rebin by ranks or by segments (write list -> read buffer).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -1372,6 +1373,8 @@ __global__ void __launch_bounds__(256) k_place_fuller(PlaceArgs a) {
         cnt = e - first;
     }
     uint32_t todo = __ballot_sync(FULL_MASK, cnt > (a.slots ? RANK_SLOTS : 1u));
+    // offsets of a scan whose wait ran out can claim bags of any length
+    if (todo && (*((volatile uint32_t*)a.err) & ERR_SPIN_TIMEOUT)) return;
     while (todo) {
         const uint32_t b = __ffs(todo) - 1;
         todo &= todo - 1u;

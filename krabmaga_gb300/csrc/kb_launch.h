@@ -250,6 +250,7 @@ struct PlaceArgs {
     uint32_t* order;
     float4* s_st;
     uint32_t* s_ids;
+    const uint32_t* err;
 };
 cudaError_t launch_count_list(const uint32_t* key, const uint8_t* dead, uint32_t n, uint32_t* hist,
                               uint32_t* slots, uint32_t ncells, uint32_t* arrival, cudaStream_t s);

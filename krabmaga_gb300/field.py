@@ -365,8 +365,8 @@ class Field2D:
         return counts[: len(q)], dig[: len(q)]
 
     def set_step_options(self, mode=0, tile_tx: int = 0, tile_ty: int = 0) -> None:
-        """Step path: 0 separate kernels (default; runs of steps on fields of
-        at most 4096 boids take one thread-block cluster), 3 separate kernels
+        """Step path: 0 separate kernels (default; fields of at most 4096
+        boids take one thread-block cluster), 3 separate kernels
         whatever the size, 2 tiled split,
         1 persistent (True/False mean 2/0); tile shape in bags (0 = automatic)."""
         mode = {True: 2, False: 0}.get(mode, mode) if isinstance(mode, bool) else int(mode)
@@ -375,7 +375,7 @@ class Field2D:
 
     def set_dense_mode(self, mode: int = L.KB_DENSE_AUTO) -> None:
         """Candidate-list walk: KB_DENSE_AUTO (by bag occupancy), _OFF (one flat
-        list, 32-bag rebin segments), _ON (per-run walk, 8-bag segments)."""
+        list, ranked rebin), _ON (per-run walk, 8-bag segments)."""
         L.call("kb_field_set_dense_mode", self._h, C.c_int32(mode))
 
     def step_path(self) -> int:
