@@ -229,7 +229,8 @@ kb_status kb_flock_step(kb_field* f, const kb_flock_params* p, uint64_t first_st
  * kernels (a plain field replays runs of 4 steps or more from CUDA graphs),
  * except that a plain field of at most 4096 boids and 4096 bags runs whole
  * steps in one 8-block thread-block cluster (shared memory, up to 1000 steps
- * per launch; a call of one step with kernel timing on does not);
+ * per launch; not a call of one step with kernel timing on, nor rings wider
+ * than one bag where the warp-per-boid kernel takes them);
  * 3 the separate kernels whatever the field's size;
  * for eligible fields (toroidal, square, jump < discretization) 2 the tiled
  * step as two launches per step (stage + rebin + force per tile, then the
@@ -246,7 +247,8 @@ kb_status kb_field_set_step_options(kb_field* f, int32_t fused, int32_t tile_tx,
  * the ranked rebin (faster for uniform ones).  Same bits either way.
  * *active (kb_field_dense_active) = the walk the next step uses. */
 kb_status kb_field_set_dense_mode(kb_field* f, int32_t mode);
-/* The path the next kb_flock_step takes: KB_PATH_* below. */
+/* The path the next kb_flock_step takes (with the last call's parameters):
+ * KB_PATH_* below. */
 #define KB_PATH_SEPARATE 0 /* separate kernels, flat candidate list */
 #define KB_PATH_FUSED 1    /* persistent fused tiles */
 #define KB_PATH_TILED 2    /* split tile step */

@@ -172,105 +172,6 @@ __global__ void __launch_bounds__(BT, MINB) k_flock_dense(ForceArgs a) {
     force_finish<STRICT, false>(a, R, i, __ldg(a.st + i), __ldg(a.ids + i), *a.step, sums.result());
 }
 
-// The agent pass of the exact query (check_circle's bag rule, field_2d.rs:
-// 934-972, then the distance): the kept bags of each column as one run, with
-// the part of it whose bags count as a whole; the three runs as one flat list.
-template <bool STRICT, int U>
-__device__ __forceinline__ void walk_exact(const ForceArgs& a, const Rep& R, float4 me4, uint32_t my,
-                                           int mi, int Mi, int mj, int Mj, Sums<STRICT>& sums) {
-    pair_t<STRICT> me;
-    pack2(me, me4.x, me4.y);
-    float ymin[3], ymax[3];  // the least and greatest squared y distance of a row's corners
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        const float nw = __fmul_rn((float)(mj + r), R.d);
-        const float n0 = __fsub_rn(nw, me4.y), n1 = __fsub_rn(fminf(__fadd_rn(nw, R.d), R.h), me4.y);
-        const float q0 = __fmul_rn(n0, n0), q1 = __fmul_rn(n1, n1);
-        ymin[r] = fminf(q0, q1);
-        ymax[r] = fmaxf(q0, q1);
-    }
-    uint32_t s[3], e[3], wl[3], wn[3];
-    bool apart = false;  // a skipped bag between two kept ones of a column
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        s[k] = e[k] = wl[k] = wn[k] = 0u;
-        if (mi + k > Mi || mj > Mj) continue;
-        const float nw = __fmul_rn((float)(mi + k), R.d);
-        const float n0 = __fsub_rn(nw, me4.x), n1 = __fsub_rn(fminf(__fadd_rn(nw, R.d), R.w), me4.x);
-        const float q0 = __fmul_rn(n0, n0), q1 = __fmul_rn(n1, n1);
-        const float xmin = fminf(q0, q1), xmax = fmaxf(q0, q1);
-        const uint32_t c = R.cell_off + (uint32_t)(mi + k) * (uint32_t)R.dh + (uint32_t)mj;
-        uint32_t o[4];
-#pragma unroll
-        for (int r = 3; r >= 0; --r) o[r] = min(__ldg(a.start + c + min(r, Mj - mj + 1)), a.n);
-#pragma unroll
-        for (int r = 2; r >= 0; --r) o[r] = min(o[r], o[r + 1]);
-        uint32_t keep = 0u, whole = 0u;
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            if (mj + r > Mj) continue;
-            if (!(__fadd_rn(xmin, ymin[r]) > R.thr)) keep |= 1u << r;
-            if (__fadd_rn(xmax, ymax[r]) <= R.thr) whole |= 1u << r;
-        }
-        apart |= keep == 5u || whole == 5u;
-        if (keep) {
-            s[k] = (keep & 1u) ? o[0] : ((keep & 2u) ? o[1] : o[2]);
-            e[k] = (keep & 4u) ? o[3] : ((keep & 2u) ? o[2] : o[1]);
-        }
-        if (whole) {
-            wl[k] = (whole & 1u) ? o[0] : ((whole & 2u) ? o[1] : o[2]);
-            wn[k] = ((whole & 4u) ? o[3] : ((whole & 2u) ? o[2] : o[1])) - wl[k];
-        }
-    }
-    auto take = [&](const Candidate<STRICT>& o, uint32_t p, bool all) {
-        const pair_t<STRICT> d = sub2(me, o.pos);
-        float dx, dy;
-        unpack2(d, dx, dy);
-        const float sq = sq_rn(dx, dy);
-        if (all || sq <= R.thr) {
-            sums.template add<true>(d, STRICT ? sq : pair_sq<STRICT>(d), o.heading, p, my);
-            sums.vec += 1u;
-            sums.count += p != my ? 1u : 0u;
-        }
-    };
-    if (apart) {  // rounding at a bag's edge: bag by bag
-#pragma unroll 1
-        for (int k = 0; mi + k <= Mi; ++k) {
-#pragma unroll 1
-            for (int r = 0; mj + r <= Mj; ++r) {
-                const int check = check_circle(mi + k, mj + r, R, me4.x, me4.y, R.radius);
-                if (check == -1) continue;
-                const uint32_t c = R.cell_off + (uint32_t)(mi + k) * (uint32_t)R.dh + (uint32_t)(mj + r);
-                const uint32_t end = min(__ldg(a.start + c + 1), a.n);
-#pragma unroll 1
-                for (uint32_t p = min(__ldg(a.start + c), end); p < end; ++p)
-                    take(load_candidate<STRICT>(a.st + p), p, check == 1);
-            }
-        }
-        return;
-    }
-    const uint32_t P1 = e[0] - s[0], P2 = P1 + (e[1] - s[1]), T = P2 + (e[2] - s[2]);
-    uint32_t p = s[0], w0 = wl[0], w1 = wn[0];
-    for (uint32_t f = 0; f < T;) {
-        Candidate<STRICT> o[U];
-        uint32_t at[U];
-        bool all[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (f == P1) { p = s[1]; w0 = wl[1]; w1 = wn[1]; }
-            if (f == P2) { p = s[2]; w0 = wl[2]; w1 = wn[2]; }
-            at[u] = p;
-            all[u] = p - w0 < w1;
-            if (u == 0 || f < T) o[u] = load_candidate<STRICT>(a.st + p);
-            ++p;
-            ++f;
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (u == 0 || f - (uint32_t)(U - u) < T) take(o[u], at[u], all[u]);
-    }
-}
-
 // How the relaxed query's lists are walked: as one flat list, run by run, or
 // by the warp's own longest list (packed replicas, whose flocks differ).
 enum Walk { WALK_FLAT, WALK_RUNS, WALK_VOTE };
@@ -285,7 +186,7 @@ __device__ __forceinline__ void ring_body(const ForceArgs& a, const Rep& R, uint
     int mi, Mi, mj, Mj;
     if (cell_range(R, me.x, me.y, R.dd, &mi, &Mi, &mj, &Mj)) {
         if (EXACT) {
-            walk_exact<STRICT, U>(a, R, me, i, mi, Mi, mj, Mj, sums);
+            walk_exact<STRICT, U>(a.st, a.start, a.n, R, me, i, mi, Mi, mj, Mj, sums);
         } else {
             pair_t<STRICT> mxy;
             pack2(mxy, me.x, me.y);

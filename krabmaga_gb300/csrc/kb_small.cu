@@ -27,7 +27,9 @@
 // between barriers, by few warps.  us per step at 300 / 1000 / 2048 / 4000 boids,
 // fast: 3.6 / 4.0 / 4.9 / 7.6, with one warp ranking the chunk in turn, every
 // record sent to all blocks and two candidates at a time without the packed
-// walk 6.5 / 7.1 / 9.3 / 13.8; strict at 1000: 4.8 against 8.6.
+// walk 6.5 / 7.1 / 9.3 / 13.8; strict at 1000: 4.8 against 8.6.  Exact query,
+// strict, 300 / 1000 / 4000: 5.3 / 5.6 / 9.9 against 17.4 / 17.9 / 25.2 bag by
+// bag with check_circle (separate kernels: 8.4 / 9.4 / 10.1).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -67,6 +69,12 @@ __device__ __forceinline__ void gather_small(const Rep& R, const float4* st, con
                                              uint32_t my_slot, Acc<STRICT>& acc) {
     int mi, Mi, mj, Mj;
     if (!cell_range(R, me.x, me.y, R.dd, &mi, &Mi, &mj, &Mj)) return;
+    if (QMODE == 1 && R.nowrap && R.dd <= 1 && my_slot != 0xFFFFFFFFu) {  // nowrap: a clamped torus
+        Sums<STRICT> sums;
+        walk_exact<STRICT, 2, false>(st, start, start[R.ncells], R, me, my_slot, mi, Mi, mj, Mj, sums);
+        acc = sums.result();
+        return;
+    }
     if (QMODE == 0 && R.toroidal && !R.cell_wrap && Mi - mi < 3) {
         if (mj > Mj) return;
         uint32_t s[3], e[3];
