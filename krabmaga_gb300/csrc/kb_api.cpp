@@ -491,12 +491,17 @@ kb_status reset_wait_state(kb_field* f) {
     return KB_OK;
 }
 
+// The arrival slots, if the buffer covers the current bag matrix.
+uint32_t* field_slots(const kb_field* f) {
+    return f->slots.n >= (size_t)f->ncells_total * RANK_SLOTS ? f->slots.p : nullptr;
+}
+
 // The arrival slots a force pass keeps for the ranked rebin; nullptr for dense
 // flocks, which rebin by segments: most of their boids share a bag with more
 // than RANK_SLOTS others, and every key of a warp would walk its source lines
 // (4M clustered boids: rebin 238 us by ranks, 160 us by 8-bag segments).
 uint32_t* rank_slots(const kb_field* f) {
-    return f->dense && f->reps.size() == 1 ? nullptr : f->slots.p;
+    return f->dense && f->reps.size() == 1 ? nullptr : field_slots(f);
 }
 
 // The general stable sort: write list -> read buffer (any list: counted here).
@@ -507,7 +512,7 @@ kb_status general_rebuild(kb_field* f) {
     if (f->hist_counted) KB_CUDA(cudaMemsetAsync(f->hist.p, 0, sizeof(uint32_t) * f->ncells_total, s));
     f->hist_counted = false;  // the scan below zeroes it
     f->slots_kept = false;
-    KB_CUDA(launch_count_list(f->wkey.p, f->wdead.p, f->wn, f->hist.p, f->slots.p, f->ncells_total, f->tid.p, s));
+    KB_CUDA(launch_count_list(f->wkey.p, f->wdead.p, f->wn, f->hist.p, field_slots(f), f->ncells_total, f->tid.p, s));
     KB_CUDA(launch_scan(f->hist.p, f->start[nxt].p, f->ncells_total, f->scan_ctl.p, f->tstate.p, f->err.p, true, s,
                         scan_wait(f)));
     PlaceArgs a{};
@@ -519,7 +524,7 @@ kb_status general_rebuild(kb_field* f) {
     a.arrival = f->tid.p;
     a.start = f->start[nxt].p;
     a.ncells = f->ncells_total;
-    a.slots = f->slots.p;
+    a.slots = field_slots(f);
     a.order = f->tsrc.p;
     a.s_st = f->rst.p;
     a.s_ids = f->rid.p;
@@ -1182,6 +1187,14 @@ kb_status field_set_reps(kb_field* f, const std::vector<Rep>& reps) {
     f->drop_graphs();
     KB_CUDA(cudaMemcpyAsync(f->d_rep.p, f->reps.data(), sizeof(Rep) * reps.size(), cudaMemcpyHostToDevice, f->stream));
     KB_CUDA(cudaStreamSynchronize(f->stream));
+    // A field whose bag capacity is above RANK_MAX_CELLS (a server: 64 slots of
+    // 2^21 bags) gets the arrival slots of the bags it uses; when they do not
+    // fit in memory it rebins by segments (28 us a step against 14 to 20 at
+    // 690,000 boids in 31 requests; 32 requests 24.4 against 21.3 ms).  Doubled, so that a batch that grows
+    // request by request allocates a few times only.
+    const size_t need = (size_t)total * RANK_SLOTS;
+    if (total <= RANK_MAX_CELLS && f->slots.n < need)
+        (void)f->slots.alloc(std::max(need, std::min<size_t>(2 * f->slots.n, (size_t)RANK_MAX_CELLS * RANK_SLOTS)));
     return build_rep_blocks(f);
 }
 

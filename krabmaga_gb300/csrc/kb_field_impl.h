@@ -59,8 +59,9 @@ struct kb_field {
     bool p_loc_differs = false;
     // step temporaries
     DevBuf<uint32_t> hist, tid, tsrc, rkey, tkey;  // rkey, tkey: the tiled steps' only
-    // arrival slots of the ranked rebin, RANK_SLOTS per bag (empty above
-    // RANK_MAX_CELLS bags: those fields rebin by segments)
+    // arrival slots of the ranked rebin, RANK_SLOTS per bag of the capacity or,
+    // where that is above RANK_MAX_CELLS bags, of the bags a batch uses (too
+    // short for the bag matrix, or empty: rebuilt by segments)
     DevBuf<uint32_t> slots;
     bool slots_kept = false;  // the last force pass left its arrivals in slots
     bool hist_counted = false;  // a force pass has counted arrivals into hist (no scan since)

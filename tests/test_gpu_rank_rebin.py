@@ -65,3 +65,23 @@ def test_packed_ranks_match_oracle(gpu, occ):
         b.step(0, 4)
         for i, r in enumerate(reps):
             assert same(b.get_replica(i), oracle_state(r.state, r.width, r.params, 4))
+
+
+@pytest.mark.parametrize("max_cells", [1 << 13, 1 << 24])
+def test_server_slots_follow_the_batch(gpu, max_cells):
+    """Slots for the whole bag capacity (2^16) and for the bags in use (a
+    capacity of 2^27): a batch that grows, grows again and shrinks."""
+    reqs = [kg.Request(n, side, D, steps, kg.FlockParams(seed=n, arith=kg.KB_ARITH_FAST), 7 + n)
+            for n, side, steps in ((300, 110.0, 40), (5000, 400.0, 21), (2000, 90.0, 33), (9, 500.0, 50))]
+    with kg.Server(max_slots=8, quantum_steps=8, max_request_boids=6000, max_request_cells=max_cells) as srv:
+        tickets = [srv.submit(reqs[0])]
+        srv.wait_idle(60.0)
+        tickets += [srv.submit(r) for r in reqs[1:]]
+        srv.wait_idle(60.0)
+        for t, r in zip(tickets, reqs):
+            f = kg.Field2D(r.side, r.side, D, True, capacity_hint=r.nboids)
+            f.set_locations(*kg.gen_uniform(r.nboids, r.side, r.side, r.init_seed, r.heading_scale))
+            f.lazy_update()
+            f.flock_step(r.params, 0, r.steps)
+            assert same(srv.result(t, r.nboids), f.get_state())
+            f.close()
