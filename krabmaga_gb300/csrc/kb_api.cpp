@@ -1190,8 +1190,9 @@ kb_status field_set_reps(kb_field* f, const std::vector<Rep>& reps) {
     // A field whose bag capacity is above RANK_MAX_CELLS (a server: 64 slots of
     // 2^21 bags) gets the arrival slots of the bags it uses; when they do not
     // fit in memory it rebins by segments (28 us a step against 14 to 20 at
-    // 690,000 boids in 31 requests; 32 requests 24.4 against 21.3 ms).  Doubled, so that a batch that grows
-    // request by request allocates a few times only.
+    // 690,000 boids in 31 requests; 32 requests 24.4 against 21.3 ms).
+    // Doubled, so that a batch that grows request by request allocates a few
+    // times only.
     const size_t need = (size_t)total * RANK_SLOTS;
     if (total <= RANK_MAX_CELLS && f->slots.n < need)
         (void)f->slots.alloc(std::max(need, std::min<size_t>(2 * f->slots.n, (size_t)RANK_MAX_CELLS * RANK_SLOTS)));

@@ -39,7 +39,7 @@ def same(got, want):
     return np.array_equal(got[0], want[0]) and np.array_equal(got[1].view(np.uint32), want[1].view(np.uint32))
 
 
-@pytest.mark.parametrize("occ", [1, 4, 5, 8, 9, 12, 13, 45])
+@pytest.mark.parametrize("occ", [1, 4, 5, 8, 9, 12, 13, 45, 131, 300])
 def test_ranks_at_row_edges_match_oracle(gpu, occ):
     side, steps = 200.0, 4
     flock = crowded(occ, side, occ)
@@ -55,7 +55,7 @@ def test_ranks_at_row_edges_match_oracle(gpu, occ):
     f.close()
 
 
-@pytest.mark.parametrize("occ", [4, 13])
+@pytest.mark.parametrize("occ", [4, 13, 140])
 def test_packed_ranks_match_oracle(gpu, occ):
     reps = []
     for i, side in enumerate((200.0, 130.0, 260.0)):
