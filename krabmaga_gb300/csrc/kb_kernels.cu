@@ -663,6 +663,10 @@ __global__ void __launch_bounds__(SCAN_THREADS)
 // the pair spreads over the chip.
 __global__ void __cluster_dims__(SCAN_CLUSTER) __launch_bounds__(1024)
     k_scan_cluster(uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint32_t n, int zero_in) {
+    // a block's shared memory may be written only once that block runs: every
+    // block says so here, and the stores below wait for it (the loads and the
+    // block scan hide the wait)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     pdl_enter();
     constexpr int ITEMS = (int)(SCAN_CLUSTER_MAX / (SCAN_CLUSTER * 1024u));
     __shared__ uint32_t s_warp[32], s_total[SCAN_CLUSTER];
@@ -688,6 +692,7 @@ __global__ void __cluster_dims__(SCAN_CLUSTER) __launch_bounds__(1024)
         if (lane >= (uint32_t)o) xi += y;
     }
     const uint32_t before = __shfl_sync(0xffffffffu, xi - x, warp), total = __shfl_sync(0xffffffffu, xi, 31);
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     if (tid < SCAN_CLUSTER) {
         uint32_t at;
         asm("mapa.shared::cluster.u32 %0, %1, %2;"
