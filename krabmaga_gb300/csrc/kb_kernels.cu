@@ -170,26 +170,25 @@ __device__ __forceinline__ void gather_candidates(const ForceArgs& a, const Rep&
         if (QMODE == 0 && clamped && Mi - mi < 5) {
             // clamped range: each column's bags mj..Mj are one contiguous
             // run; fetch every run's bounds before touching candidates
-            if (mj <= Mj) {
-                // a one-bag ring (the common case) as one flat list; the wider
-                // two-bag ring out of line
-                if (Mi - mi < 3)
-                    columns_flat3<STRICT, DENSE>(a, R, mi, Mi, mj, Mj, me, my_id, acc, my_slot);
-                else columns_runs_5(a, R, mi, Mi, mj, Mj, me, my_id, acc);
-            }
+            // a one-bag ring (the common case) as one flat list; the wider
+            // two-bag ring out of line
+            if (Mi - mi < 3)
+                columns_flat3<STRICT, DENSE>(a, R, mi, Mi, mj, Mj, me, my_id, acc, my_slot);
+            else columns_runs_5(a, R, mi, Mi, mj, Mj, me, my_id, acc);
         } else {
-            for (int ci = mi; ci <= Mi; ++ci) {
-                const int bx = t_transform(ci, R.max_x);
+            // counted: a line number may be the greatest i32
+            const uint32_t ni = (uint32_t)Mi - (uint32_t)mi, nj = (uint32_t)Mj - (uint32_t)mj;
+            for (uint32_t u = 0; u <= ni; ++u) {
+                const int bx = t_transform((int)((uint32_t)mi + u), R.max_x);
                 const uint32_t colbase = R.cell_off + (uint32_t)bx * (uint32_t)R.dh;
                 if (QMODE == 0 && clamped) {
-                    if (mj > Mj) continue;
                     const uint32_t e = min(__ldg(a.start + colbase + Mj + 1), a.n);
                     accumulate_run(R, a.st, a.ids, min(__ldg(a.start + colbase + mj), e), e, me,
                                    my_id, acc);
                     continue;
                 }
-                for (int cj = mj; cj <= Mj; ++cj) {
-                    const int by = t_transform(cj, R.max_y);
+                for (uint32_t v = 0; v <= nj; ++v) {
+                    const int by = t_transform((int)((uint32_t)mj + v), R.max_y);
                     const uint32_t c = colbase + (uint32_t)by;
                     const uint32_t e = min(__ldg(a.start + c + 1), a.n);
                     const uint32_t s = min(__ldg(a.start + c), e);
@@ -1517,14 +1516,14 @@ __device__ __forceinline__ bool query_ring(const QueryArgs& a, float2 p, int mi,
         const uint32_t c = R.cell_off + (uint32_t)(mi + k) * (uint32_t)R.dh + (uint32_t)mj;
 #pragma unroll
         for (int r = 0; r < 4; ++r)
-            o[k][r] = mi + k <= Mi && mj <= Mj ? __ldg(a.start + c + min(r, Mj - mj + 1)) : 0u;
+            o[k][r] = mi + k <= Mi ? __ldg(a.start + c + min(r, Mj - mj + 1)) : 0u;
     }
     uint32_t s[3], e[3], wl[3], wn[3];
     bool apart = false;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         s[k] = e[k] = wl[k] = wn[k] = 0u;
-        if (mi + k > Mi || mj > Mj) continue;
+        if (mi + k > Mi) continue;
         uint32_t keep = 7u, whole = 7u;
         if (KIND == 1) {
             const float nw = __fmul_rn((float)(mi + k), R.d);
@@ -1613,10 +1612,12 @@ __global__ void k_query(QueryArgs a) {
                query_ring<KIND>(a, p, mi, Mi, mj, Mj, off, fill, &cnt, &dig)) {
         // done
     } else {
-        for (int ci = mi; ci <= Mi; ++ci) {
-            const int bx = t_transform(ci, R.max_x);
-            for (int cj = mj; cj <= Mj; ++cj) {
-                const int by = t_transform(cj, R.max_y);
+        // counted: a line number may be the greatest i32
+        const uint32_t ni = (uint32_t)Mi - (uint32_t)mi, nj = (uint32_t)Mj - (uint32_t)mj;
+        for (uint32_t u = 0; u <= ni; ++u) {
+            const int bx = t_transform((int)((uint32_t)mi + u), R.max_x);
+            for (uint32_t v = 0; v <= nj; ++v) {
+                const int by = t_transform((int)((uint32_t)mj + v), R.max_y);
                 const uint32_t c = R.cell_off + (uint32_t)bx * (uint32_t)R.dh + (uint32_t)by;
                 const uint32_t s = a.start[c], e = a.start[c + 1];
                 if (s == e) continue;

@@ -33,7 +33,7 @@ __device__ __forceinline__ void relaxed_runs(const ForceArgs& a, const Rep& R, i
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         r.s[k] = r.e[k] = 0u;
-        if (mi + k <= Mi && mj <= Mj) {
+        if (mi + k <= Mi) {
             const uint32_t c = R.cell_off + (uint32_t)(mi + k) * (uint32_t)R.dh;
             r.e[k] = min(__ldg(a.start + c + Mj + 1), a.n);
             r.s[k] = min(__ldg(a.start + c + mj), r.e[k]);

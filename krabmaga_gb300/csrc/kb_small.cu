@@ -76,7 +76,6 @@ __device__ __forceinline__ void gather_small(const Rep& R, const float4* st, con
         return;
     }
     if (QMODE == 0 && R.toroidal && !R.cell_wrap && Mi - mi < 3) {
-        if (mj > Mj) return;
         uint32_t s[3], e[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -109,7 +108,6 @@ __device__ __forceinline__ void gather_small(const Rep& R, const float4* st, con
         return;
     }
     if (QMODE == 0 && R.toroidal && !R.cell_wrap) {  // wider rings: a run per column
-        if (mj > Mj) return;
         for (int ci = mi; ci <= Mi; ++ci) {
             const uint32_t colbase = (uint32_t)ci * (uint32_t)R.dh;
             const uint32_t e = start[colbase + (uint32_t)Mj + 1u];

@@ -199,7 +199,7 @@ __device__ __forceinline__ void walk_exact(const float4* st, const uint32_t* sta
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         s[k] = e[k] = wl[k] = wn[k] = 0u;
-        if (mi + k > Mi || mj > Mj) continue;
+        if (mi + k > Mi) continue;
         const float nw = __fmul_rn((float)(mi + k), R.d);
         const float n0 = __fsub_rn(nw, me4.x), n1 = __fsub_rn(fminf(__fadd_rn(nw, R.d), R.w), me4.x);
         const float q0 = __fmul_rn(n0, n0), q1 = __fmul_rn(n1, n1);

@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(32 * WIDE_WARPS) k_flock_wide(ForceArgs a) {
     float acc = 0.f;  // lane c < 6: sum c
     uint32_t vec = 0, count = 0;
     int mi, Mi, mj, Mj;
-    if (cell_range(R, me.x, me.y, R.dd, &mi, &Mi, &mj, &Mj) && mj <= Mj) {
+    if (cell_range(R, me.x, me.y, R.dd, &mi, &Mi, &mj, &Mj)) {
 #pragma unroll 1
         for (int col = mi; col <= Mi; col += 32) {
             const int bx = col + (int)lane;
