@@ -275,9 +275,11 @@ __global__ void __launch_bounds__(T, 1) k_small_steps(SmallArgs a) {
     if (t < 2u * SMALL_CTAS) line[t / SMALL_CTAS][t % SMALL_CTAS] = 0u;
     if (t == 0) {
         s_err = 0u;
-        // records go to every block where a query can wrap, and from the step
-        // on in which a position fell outside the matrix
-        s_all = R.toroidal && !R.cell_wrap ? 0u : 1u;
+        // records go to every block where a query can wrap, where birds stand
+        // beyond the height (y wraps with the width), in bags of other columns
+        // than their positions', and from the step on in which a position fell
+        // outside the matrix
+        s_all = R.toroidal && !R.cell_wrap && R.w <= R.h ? 0u : 1u;
     }
     // a thread writes to one other block: keys, records and ids of block t % 8
     static_assert(T % SMALL_CTAS == 0 && SMALL_CTAS == 8, "one target block per thread");
