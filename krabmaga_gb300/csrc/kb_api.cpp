@@ -131,8 +131,11 @@ void set_rep_params(Rep* R, const kb_flock_params* p) {
     // With the clamped (toroidal) cell range every candidate lies within
     // (dd+1)*d of the boid, so toroidal_distance's |a-b| <= dim/2 test holds
     // whenever (dd+1)*d stays clear of half the side.
+    // A bird's y wraps with the width (bird.rs:147): where the last row below the
+    // width lies past the matrix, a bird's bag is one of another column, and its
+    // neighbours by bag may stand anywhere.
     const double reach = ((double)std::max(R->dd, 0) + 1.0) * (double)R->d;
-    R->nowrap = (R->toroidal && !R->cell_wrap &&
+    R->nowrap = (R->toroidal && !R->cell_wrap && as_i32(std::floor(R->w / R->d)) <= R->max_y &&
                  reach * 1.01 + 1e-3 < 0.5 * (double)std::min(R->w, R->h)) ? 1 : 0;
     // A move of at most |jump| wraps to line 0 only from x > w - |jump|, i.e.
     // from lines >= floor((w - |jump|)/d); one line lower covers the f32

@@ -45,7 +45,7 @@ struct Rep {
     int32_t dd;             // floor(radius/d) (field_2d.rs:488), -1 when radius <= 0
     int32_t qmode;          // 0 relax, 1 exact
     uint32_t seed_lo, seed_hi;
-    int32_t nowrap;         // 1: no candidate pair can straddle the seam ((dd+1)*d < min(w,h)/2)
+    int32_t nowrap;         // 1: no candidate pair can straddle the seam (set_rep_params)
     uint32_t origin_lo, origin_hi;  // global step at which this replica's step 0 ran
     int32_t seam;           // first line from which a one-step move can wrap to line 0
     float inv_d;            // fl(1/d), for the exact fast discretisation

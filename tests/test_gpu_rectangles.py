@@ -55,3 +55,79 @@ def test_cluster_sends_what_wide_rings_read(gpu, w, h, kind, repeat):
     assert f.step_path() == kg.KB_PATH_SMALL
     assert same(f.get_state(), oracle_after(w, h, 1.0, birds, p, 25))
     f.close()
+
+
+D = float(np.float32(10.0) / np.float32(1.5))
+SHAPES = [(100.0, 60.0), (60.0, 100.0), (240.0, 200.0), (200.0, 240.0), (102.0, 100.0)]
+
+
+@pytest.mark.parametrize("kind", QUERIES)
+@pytest.mark.parametrize("w,h", SHAPES)
+@pytest.mark.parametrize("mode", [0, 3])  # whole steps in the cluster, the separate kernels
+@pytest.mark.parametrize("d,dense", [(D, False), (4.0, False), (1.5, False), (D, True)])
+def test_steps_match_oracle(gpu, mode, w, h, kind, d, dense):
+    birds = flock(900, w, h, int(w))
+    p = kg.FlockParams(seed=4, arith=kg.KB_ARITH_STRICT, query_mode=kind)
+    f = plain(w, h, d, birds, mode)
+    f.set_dense_mode(kg.KB_DENSE_ON if dense else kg.KB_DENSE_OFF)
+    f.flock_step(p, 0, 1)
+    f.flock_step(p, 1, 14)
+    assert same(f.get_state(), oracle_after(w, h, d, birds, p, 15))
+    f.close()
+
+
+@pytest.mark.parametrize("kind", QUERIES)
+@pytest.mark.parametrize("w,h", [(480.0, 400.0), (400.0, 480.0)])
+def test_larger_flocks_match_oracle(gpu, w, h, kind):
+    birds = flock(6000, w, h, 1)
+    p = kg.FlockParams(seed=4, arith=kg.KB_ARITH_STRICT, query_mode=kind)
+    f = plain(w, h, D, birds)
+    f.flock_step(p, 0, 10)
+    assert same(f.get_state(), oracle_after(w, h, D, birds, p, 10))
+    f.close()
+
+
+@pytest.mark.parametrize("kind", QUERIES)
+def test_fast_arithmetic_on_both_paths_is_the_same(gpu, kind):
+    w, h = 200.0, 130.0
+    birds = flock(900, w, h, 2)
+    p = kg.FlockParams(seed=4, arith=kg.KB_ARITH_FAST, query_mode=kind)
+    out = []
+    for mode in (0, 3):
+        f = plain(w, h, D, birds, mode)
+        f.flock_step(p, 0, 15)
+        out.append(f.get_state())
+        f.close()
+    assert same(*out)
+
+
+@pytest.mark.parametrize("kind", QUERIES)
+@pytest.mark.parametrize("d", [D, 4.0])
+def test_packed_rectangles_match_oracle(gpu, kind, d):
+    reps = []
+    for i, (w, h) in enumerate(SHAPES):
+        p = kg.FlockParams(seed=i, arith=kg.KB_ARITH_STRICT, query_mode=kind)
+        reps.append(kg.Replica(w, h, d, p, flock(500 + i, w, h, 10 + i)))
+    with kg.Batch(reps) as b:
+        b.step(0, 12)
+        for i, r in enumerate(reps):
+            assert same(b.get_replica(i), oracle_after(r.width, r.height, d, r.state, r.params, 12))
+
+
+@pytest.mark.parametrize("kind", QUERIES)
+@pytest.mark.parametrize("w,h", SHAPES)
+def test_queries_after_steps_match_oracle(gpu, w, h, kind):
+    birds = flock(900, w, h, 7)
+    p = kg.FlockParams(seed=4, arith=kg.KB_ARITH_STRICT)
+    f = plain(w, h, D, birds)
+    f.flock_step(p, 0, 15)
+    o = oracle.OracleField(w, h, D, True)
+    o.set_many(*birds)
+    o.lazy_update()
+    o.flock_run(oracle.params_from(p), 0, 15)
+    r = np.random.default_rng(1)
+    q = np.concatenate([f.get_state()[1][:, :2], r.uniform(-8.0, max(w, h) + 8.0, (300, 2))]).astype(np.float32)
+    counts, ids = f.neighbor_lists(kind, 10.0, q)
+    want = o.neighbor_lists(kind, 10.0, q)
+    assert np.array_equal(counts, want[0]) and np.array_equal(ids, want[1])
+    f.close()
