@@ -70,6 +70,13 @@ int64_t host_bag_index(const Rep& R, float x, float y) {
     return idx;
 }
 
+// Whether a position's own column and row are lines of the matrix.  The bag
+// index of another one can still lie inside it: a bag of some other column.
+bool host_inside(const Rep& R, float x, float y) {
+    const int32_t cx = as_i32(std::floor(x / R.d)), cy = as_i32(std::floor(y / R.d));
+    return cx >= 0 && cx <= R.max_x && cy >= 0 && cy <= R.max_y;
+}
+
 bool make_rep_geometry(float w, float h, float d, int toroidal, Rep* R, std::string* why,
                        int cell_wrap) {
     if (!(std::isfinite(w) && std::isfinite(h) && std::isfinite(d)) || w <= 0.f || h <= 0.f ||
@@ -417,15 +424,15 @@ kb_status flush_pending(kb_field* f) {
     return KB_OK;
 }
 
-kb_status read_u32(kb_field* f, const uint32_t* dptr, uint32_t* out) {
+kb_status read_u32(kb_field* f, const uint32_t* dptr, uint32_t* out, uint32_t words) {
     if (f->occ_host) {  // through pinned memory: no staging copy
         uint32_t* w = reinterpret_cast<uint32_t*>(f->occ_host + PIN_WORD);
-        KB_CUDA(cudaMemcpyAsync(w, dptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, f->stream));
+        KB_CUDA(cudaMemcpyAsync(w, dptr, sizeof(uint32_t) * words, cudaMemcpyDeviceToHost, f->stream));
         KB_CUDA(cudaStreamSynchronize(f->stream));
-        *out = *w;
+        std::copy(w, w + words, out);
         return KB_OK;
     }
-    KB_CUDA(cudaMemcpyAsync(out, dptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, f->stream));
+    KB_CUDA(cudaMemcpyAsync(out, dptr, sizeof(uint32_t) * words, cudaMemcpyDeviceToHost, f->stream));
     KB_CUDA(cudaStreamSynchronize(f->stream));
     return KB_OK;
 }
@@ -581,10 +588,8 @@ kb_status fast_rebuild(kb_field* f, bool bump_step, bool stencil) {
 // small plain field the warp-per-boid one (ForceArgs::wide).
 bool ring_ok(const kb_field* f, bool* wide) {
     *wide = false;
-    if (!f->ids_unique || f->rn > (1u << 26)) return false;
-    // objects set apart from their own positions: the exact query's distances
-    // can wrap although no ring does
-    if (!f->layout_is_positions && f->reps[0].qmode != KB_QUERY_RELAX) return false;
+    // objects apart from their bags: distances can wrap although no ring does
+    if (!f->ids_unique || f->rn > (1u << 26) || !f->layout_is_positions) return false;
     bool one = true;
     for (const Rep& R : f->reps) {
         if (!R.toroidal || R.cell_wrap || !R.nowrap) return false;
@@ -594,11 +599,20 @@ bool ring_ok(const kb_field* f, bool* wide) {
     return one;
 }
 
+// A plain field's record for the force kernels: where objects stand apart from
+// their bags, a pair of neighbouring bags may straddle the seam.
+Rep force_rep(const kb_field* f) {
+    Rep R = f->reps[0];
+    if (!f->layout_is_positions) R.nowrap = 0;
+    return R;
+}
+
 kb_status enqueue_force(kb_field* f, const kb_flock_params* p) {
     ForceArgs a{};
     a.reps = f->d_rep.p;
     a.nrep = nrep(f);
-    a.rep0 = f->reps[0];
+    a.rep0 = force_rep(f);
+    a.apart = f->layout_is_positions ? 0 : 1;
     a.st = f->rst.p;
     a.ids = f->rid.p;
     a.start = f->start[f->cur].p;
@@ -1292,7 +1306,7 @@ kb_status kb_field_set_object_location(kb_field* f, uint32_t id, const float pos
     f->p_st.push_back(make_float4(pos[0], pos[1], last_d[0], last_d[1]));
     f->p_id.push_back(id);
     f->p_key.push_back((uint32_t)idx);
-    if (host_bag_index(f->rep, pos[0], pos[1]) != idx) f->p_loc_differs = true;
+    if (host_bag_index(f->rep, pos[0], pos[1]) != idx || !host_inside(f->rep, pos[0], pos[1])) f->p_loc_differs = true;
     if (!f->density_check) f->nagents += 1;
     f->w_from_compute = false;
     return KB_OK;
@@ -1319,11 +1333,12 @@ kb_status kb_field_set_locations(kb_field* f, size_t n, const uint32_t* ids, con
     KB_CUDA(cudaMemcpyAsync(sxy, xy, sizeof(float2) * m, cudaMemcpyHostToDevice, f->stream));
     KB_CUDA(cudaMemcpyAsync(sdxy, dxy, sizeof(float2) * m, cudaMemcpyHostToDevice, f->stream));
     KB_CUDA(cudaMemcpyAsync(f->wid.p + f->wn, ids, sizeof(uint32_t) * m, cudaMemcpyHostToDevice, f->stream));
-    KB_CUDA(cudaMemsetAsync(f->small.p, 0xFF, sizeof(uint32_t), f->stream));
+    KB_CUDA(cudaMemsetAsync(f->small.p, 0xFF, 2 * sizeof(uint32_t), f->stream));
     KB_CUDA(launch_pack_locations(f->rep, sxy, sdxy, m, f->wst.p + f->wn, f->wkey.p + f->wn,
                                   f->wdead.p + f->wn, f->small.p, f->stream));
-    uint32_t bad = 0;
-    if ((st = read_u32(f, f->small.p, &bad))) return st;
+    uint32_t found[2] = {0, 0};  // the first bad object, the first one outside the matrix's lines
+    if ((st = read_u32(f, f->small.p, found, 2))) return st;
+    const uint32_t bad = found[0];
     if (bad != 0xFFFFFFFFu) {  // the write list is left as it was
         const size_t i = bad;
         if (!(std::isfinite(xy[2 * i]) && std::isfinite(xy[2 * i + 1]) &&
@@ -1334,6 +1349,7 @@ kb_status kb_field_set_locations(kb_field* f, size_t n, const uint32_t* ids, con
         return fail(KB_ERR_RANGE, buf);
     }
     f->wn += m;
+    if (found[1] != 0xFFFFFFFFu) f->layout_is_positions = false;
     if (!f->density_check) f->nagents += n;
     f->w_from_compute = false;
     return KB_OK;
@@ -1997,7 +2013,7 @@ kb_status kb_flock_compute_agents(kb_field* f, const kb_flock_params* p, uint64_
     ForceArgs a{};
     a.reps = f->d_rep.p;
     a.nrep = 1;
-    a.rep0 = f->reps[0];
+    a.rep0 = force_rep(f);
     a.st = f->rst.p;
     a.ids = f->rid.p;
     a.start = f->start[f->cur].p;
@@ -2052,17 +2068,19 @@ kb_status kb_field_set_states_device(kb_field* f, size_t n, const uint32_t* ids_
     if ((st = grow(f, f->wn + (uint32_t)n))) return st;
     const uint32_t m = (uint32_t)n;
     KB_CUDA(cudaMemcpyAsync(f->wid.p + f->wn, ids_dev, sizeof(uint32_t) * m, cudaMemcpyDeviceToDevice, f->stream));
-    KB_CUDA(cudaMemsetAsync(f->small.p, 0xFF, sizeof(uint32_t), f->stream));
+    KB_CUDA(cudaMemsetAsync(f->small.p, 0xFF, 2 * sizeof(uint32_t), f->stream));
     KB_CUDA(launch_pack_states(f->rep, reinterpret_cast<const float4*>(states_dev), m, f->wst.p + f->wn,
                                f->wkey.p + f->wn, f->wdead.p + f->wn, f->small.p, f->stream));
-    uint32_t bad = 0;
-    if ((st = read_u32(f, f->small.p, &bad))) return st;
+    uint32_t found[2] = {0, 0};  // the first bad object, the first one outside the matrix's lines
+    if ((st = read_u32(f, f->small.p, found, 2))) return st;
+    const uint32_t bad = found[0];
     if (bad != 0xFFFFFFFFu) {  // the write list is left as it was
         char buf[128];
         std::snprintf(buf, sizeof buf, "object %u: non-finite record or location outside the bag matrix", bad);
         return fail(KB_ERR_RANGE, buf);
     }
     f->wn += m;
+    if (found[1] != 0xFFFFFFFFu) f->layout_is_positions = false;
     if (!f->density_check) f->nagents += n;
     f->w_from_compute = false;
     return KB_OK;
@@ -2097,7 +2115,7 @@ kb_status kb_flock_next_states_device(kb_field* f, const kb_flock_params* p, uin
     ForceArgs a{};
     a.reps = f->d_rep.p;
     a.nrep = 1;
-    a.rep0 = f->reps[0];
+    a.rep0 = force_rep(f);
     a.st = f->rst.p;
     a.ids = f->rid.p;
     a.start = f->start[f->cur].p;

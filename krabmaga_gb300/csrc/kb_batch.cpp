@@ -118,6 +118,7 @@ kb_status kb_batch_set_replica(kb_batch* b, uint32_t r, size_t n, const uint32_t
         f->p_st.push_back(make_float4(xy[2 * i], xy[2 * i + 1], dxy[2 * i], dxy[2 * i + 1]));
         f->p_id.push_back(ids[i]);
         f->p_key.push_back(R.cell_off + (uint32_t)idx);
+        if (!host_inside(R, xy[2 * i], xy[2 * i + 1])) f->p_loc_differs = true;
     }
     b->have[r] = 1;
     return KB_OK;
@@ -157,6 +158,12 @@ kb_status kb_batch_step(kb_batch* b, uint64_t first_step, uint32_t nsteps, uint3
     kb_status st;
     KB_CUDA(launch_set_u64(f->dstep.p, first_step, f->stream));
     f->dstep_host = ~0ull;
+    if (!f->layout_is_positions) {  // objects outside their matrix's lines: one general step brings them in
+        if ((st = grow(f, f->rn))) return st;
+        if ((st = enqueue_steps(f, p, 1, false))) return st;
+        f->layout_is_positions = true;
+        if (--nsteps == 0) return KB_OK;
+    }
     if (!fused_eligible(f, p)) {
         if ((st = materialize(f))) return st;
         if ((st = grow(f, f->rn))) return st;
@@ -394,14 +401,15 @@ static kb_status batch_repack(kb_batch* b, std::vector<Rep> reps, const std::vec
         KB_CUDA(cudaMemcpyAsync(sxy, xy, sizeof(float2) * m, cudaMemcpyHostToDevice, f->stream));
         KB_CUDA(cudaMemcpyAsync(sxy + m, dxy, sizeof(float2) * m, cudaMemcpyHostToDevice, f->stream));
         KB_CUDA(cudaMemcpyAsync(f->wid.p + at, ids, sizeof(uint32_t) * m, cudaMemcpyHostToDevice, f->stream));
-        KB_CUDA(cudaMemsetAsync(f->small.p, 0xFF, sizeof(uint32_t), f->stream));
+        KB_CUDA(cudaMemsetAsync(f->small.p, 0xFF, 2 * sizeof(uint32_t), f->stream));
         KB_CUDA(launch_pack_locations(R, sxy, sxy + m, m, f->wst.p + at, f->wkey.p + at, f->wdead.p + at,
                                       f->small.p, f->stream));
-        uint32_t bad = 0;
-        if ((st = read_u32(f, f->small.p, &bad))) return st;
-        if (bad != 0xFFFFFFFFu)
-            return fail(KB_ERR_RANGE, "new replica: object " + std::to_string(bad) +
+        uint32_t found[2] = {0, 0};
+        if ((st = read_u32(f, f->small.p, found, 2))) return st;
+        if (found[0] != 0xFFFFFFFFu)
+            return fail(KB_ERR_RANGE, "new replica: object " + std::to_string(found[0]) +
                                           " outside its bag matrix on the device");
+        if (found[1] != 0xFFFFFFFFu) f->layout_is_positions = false;
     }
     f->wn = (uint32_t)boids;
     f->w_from_compute = false;
@@ -410,7 +418,6 @@ static kb_status batch_repack(kb_batch* b, std::vector<Rep> reps, const std::vec
     f->p_st.clear(); f->p_id.clear(); f->p_key.clear();
     if ((st = general_rebuild(f))) return st;
     f->wn = 0;
-    f->layout_is_positions = true;
     if ((st = load_facts(f, (uint32_t)boids))) return st;
     f->rn = (uint32_t)boids;
     b->have.assign(reps.size(), 1);

@@ -53,7 +53,7 @@ struct kb_field {
     uint32_t wn = 0;
     bool w_from_compute = false;   // write list == one flock pass over the read buffer
     bool w_has_dead = false;
-    bool layout_is_positions = true;  // every stored bag == discretize(own pos)
+    bool layout_is_positions = true;  // every stored bag is at its position's own column and row
     std::vector<float4> p_st;
     std::vector<uint32_t> p_id, p_key;
     bool p_loc_differs = false;
@@ -215,6 +215,7 @@ namespace kb {
 extern thread_local std::string g_last_error;  // kb_last_error()'s message for this thread
 // Host copy of discretize + bag index (field_2d.rs:328-339): -1 outside the matrix.
 int64_t host_bag_index(const Rep& R, float x, float y);
+bool host_inside(const Rep& R, float x, float y);
 // Field2D::new geometry (field_2d.rs:304-322) into R; false with *why on bad input.
 bool make_rep_geometry(float w, float h, float d, int toroidal, Rep* R, std::string* why,
                        int cell_wrap = KB_CELL_WRAP_CLAMP);
@@ -266,5 +267,5 @@ void set_ids_unique(kb_field* f, bool u);
 // Reset the control words of the bounded-wait protocols (after a timeout).
 kb_status reset_wait_state(kb_field* f);
 // Synchronous reads: one device word; the device error word as a status.
-kb_status read_u32(kb_field* f, const uint32_t* dptr, uint32_t* out);
+kb_status read_u32(kb_field* f, const uint32_t* dptr, uint32_t* out, uint32_t words = 1);
 kb_status check_flags(kb_field* f);

@@ -247,6 +247,10 @@ __global__ void __launch_bounds__(BT, (MULTI ? KB_FORCE_MINB_MULTI : KB_FORCE_MI
         const uint2 e = a.blk[blockIdx.x];
         load_rep_shared(&sR, a.reps + e.x);
         __syncthreads();
+        if (a.apart) {
+            if (threadIdx.x == 0) sR.nowrap = 0;
+            __syncthreads();
+        }
         const uint32_t k = e.y + threadIdx.x;
         if (k >= sR.boid_off + sR.nboids) return;
         force_body<STRICT, QMODE, false>(a, sR, k);
@@ -1855,6 +1859,12 @@ __global__ void k_dup_check(const Rep* __restrict__ reps, int32_t nrep, const ui
     *dup = 1u;  // no free slot found (cannot happen at half occupancy): be conservative
 }
 
+// The first object whose own column or row is no line of the matrix.
+__device__ __forceinline__ void note_outside(const Rep& R, float x, float y, uint32_t i, uint32_t* first) {
+    const int32_t cx = disc(x, R), cy = disc(y, R);
+    if (cx < 0 || cx > R.max_x || cy < 0 || cy > R.max_y) atomicMin(first, i);
+}
+
 __global__ void k_pack_locations(Rep R, const float2* __restrict__ xy, const float2* __restrict__ dxy,
                                  uint32_t n, float4* __restrict__ out_st, uint32_t* __restrict__ out_key,
                                  uint8_t* __restrict__ out_dead, uint32_t* bad) {
@@ -1866,6 +1876,7 @@ __global__ void k_pack_locations(Rep R, const float2* __restrict__ xy, const flo
         atomicMin(bad, i);
         return;
     }
+    note_outside(R, p.x, p.y, i, bad + 1);
     out_st[i] = make_float4(p.x, p.y, d.x, d.y);
     out_key[i] = R.cell_off + (uint32_t)idx;
     out_dead[i] = 0;
@@ -1883,6 +1894,7 @@ __global__ void k_pack_states(Rep R, const float4* __restrict__ st, uint32_t n,
         atomicMin(bad, i);
         return;
     }
+    note_outside(R, v.x, v.y, i, bad + 1);
     out_st[i] = v;
     out_key[i] = R.cell_off + (uint32_t)idx;
     out_dead[i] = 0;

@@ -81,6 +81,7 @@ struct ForceArgs {
     uint32_t* slots;
     uint32_t ncells;  // bags over all replicas (the second row of a.slots starts behind them)
     uint32_t* err;
+    int32_t apart;  // objects may stand apart from their bags: no replica's nowrap holds
     int32_t check_moves;  // flag moves the stencil-gather rebin cannot follow
     // several replicas: one block per entry {replica, first boid}; no block
     // spans two replicas (built by the host with the replica table)
@@ -224,8 +225,9 @@ cudaError_t launch_moments(const Rep* reps, uint32_t nrep, const uint32_t* start
 
 // Bulk set_object_location on the device: n objects at their own positions
 // (xy and dxy as float2 arrays) appended to the write list as records, bag
-// keys and live marks; *bad takes the smallest index of an object with a
-// non-finite value or a location outside the bag matrix (~0u when none).
+// keys and live marks; bad[0] takes the smallest index of an object with a
+// non-finite value or a location outside the bag matrix, bad[1] that of one
+// whose own column or row is no line of the matrix (~0u when none).
 cudaError_t launch_pack_locations(const Rep& rep, const float2* xy, const float2* dxy, uint32_t n,
                                   float4* out_st, uint32_t* out_key, uint8_t* out_dead,
                                   uint32_t* bad, cudaStream_t s);
