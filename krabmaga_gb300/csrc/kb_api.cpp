@@ -627,9 +627,11 @@ kb_status enqueue_force(kb_field* f, const kb_flock_params* p) {
     f->slots_kept = a.slots != nullptr;
     a.err = f->err.p;
     // The fast rebin is used only when |jump| * 1.001 < d, so no boid can
-    // leave the 3x3 stencil; the rebin's own count check (every bag gathers
-    // exactly its counted arrivals) reports any miss.  The per-boid move check
-    // only names the cause, at two extra discretisations per boid.
+    // leave the 3x3 stencil, and it reports a miss itself: the segments compare
+    // what a bag gathered with its count; the ranks place every arrival that has
+    // a slot wherever it came from, and an arrival of a fuller bag looks for its
+    // own place among the bag's source lines.  The per-boid move check would
+    // take two more discretisations per boid.
     a.check_moves = 0;
     a.blk = f->nblk_force ? f->blk_force.p : nullptr;
     a.nblk = f->nblk_force;

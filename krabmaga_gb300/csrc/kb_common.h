@@ -22,7 +22,7 @@ enum : uint32_t {
     // which check raised a rebin miss (set together with ERR_REBIN_MISS)
     ERR_MISS_GATHER = 0x10u,   // a bag gathered a different count than its offsets say
     ERR_MISS_OUTSIDE = 0x20u,  // a boid sits outside the bag its slot belongs to
-    ERR_MISS_MOVE = 0x40u,     // a boid moved further than the neighbouring bag
+    ERR_MISS_MOVE = 0x40u,     // a boid moved further than the neighbouring bag (seen by the ranked rebin)
     ERR_MISS_TILE = 0x80u,     // a tile was refused (ring wider than the layout)
     ERR_MISS_MATERIALIZE = 0x100u,  // the standalone rebin found a different count
 };

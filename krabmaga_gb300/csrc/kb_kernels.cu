@@ -1116,13 +1116,16 @@ __global__ void __launch_bounds__(32 * REBIN_SEG_WARPS, MULTI ? KB_REBIN_MINB_MU
 // 20.6, 64 condensing replicas 58.3 against 57.4 ms).  Every lane of the warp calls it with its
 // entry i (over: the entry's bag is a fuller one).  Out of line and after the
 // others are written, so that it costs them no registers.
+// The source lines hold every arrival unless one has moved past them.  Each
+// entry looks for its own place in its bag's lines; one that is not there would
+// be missing from the other arrivals' counts, and raises the error word.
 template <bool MULTI>
 __device__ __noinline__ void place_by_lines(const RebinArgs& a, bool over, uint32_t i) {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t key = 0, first = 0, rank = 0;
     // an interior bag's source columns, entries [s, e) each, ascending
     uint32_t s0 = 0, e0 = 0, s1 = 0, e1 = 0, s2 = 0, e2 = 0;
-    bool inner = false;
+    bool inner = false, seen = a.any_move != 0;
     if (over) {
         key = __ldcg(a.key + i);
         first = __ldg(a.start_next + key);
@@ -1137,6 +1140,7 @@ __device__ __noinline__ void place_by_lines(const RebinArgs& a, bool over, uint3
                 e0 = min(__ldg(c - dh + 2), a.n), s0 = min(__ldg(c - dh - 1), e0);
                 e1 = min(__ldg(c + 2), a.n), s1 = min(__ldg(c - 1), e1);
                 e2 = min(__ldg(c + dh + 2), a.n), s2 = min(__ldg(c + dh - 1), e2);
+                seen = i - s0 < e0 - s0 || i - s1 < e1 - s1 || i - s2 < e2 - s2;
             }
         }
     }
@@ -1180,6 +1184,7 @@ __device__ __noinline__ void place_by_lines(const RebinArgs& a, bool over, uint3
         const uint32_t Xu = div_dh(local, R);
         const int X = (int)Xu, Y = (int)(local - Xu * (uint32_t)R.dh);
         auto count = [&](uint32_t s, uint32_t end) {
+            seen |= mine && i - s < end - s;
             const uint32_t e = min(end, last);
 #pragma unroll 2
             for (uint32_t p = s; p < e; p += 32u) {
@@ -1212,6 +1217,7 @@ __device__ __noinline__ void place_by_lines(const RebinArgs& a, bool over, uint3
             }
         }
     }
+    if (over && !seen) atomicOr(a.err, ERR_REBIN_MISS | ERR_MISS_MOVE);
     if (over && first + rank < a.n) {
         a.s_st[first + rank] = __ldcg(a.a_st + i);
         a.s_ids[first + rank] = __ldcg(a.a_ids + i);
