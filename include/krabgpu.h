@@ -356,6 +356,8 @@ kb_status kb_debug_allocation_counts(uint64_t* allocs, uint64_t* frees);
  * then return KB_ERR_OOM, and the request server fails the requests of the
  * epoch that met it and carries on with the next ones. */
 kb_status kb_debug_fail_allocations(uint32_t count);
+/* The same after `skip` more allocations that are made as usual. */
+kb_status kb_debug_fail_allocations_after(uint32_t skip, uint32_t count);
 
 /* ------------------------------------------------------ batched replicas */
 /* Many independent Flockers simulations (the model-exploration workload of

@@ -22,7 +22,7 @@ namespace kb {
 thread_local std::string g_last_error;
 
 std::atomic<unsigned long long> g_dev_allocs{0}, g_dev_frees{0};
-std::atomic<long long> g_fail_allocs{0};
+std::atomic<long long> g_fail_allocs{0}, g_fail_skip{0};
 
 kb_status fail(kb_status code, const std::string& msg) {
     g_last_error = msg;
@@ -198,6 +198,32 @@ bool fast_rebin_ok(const Rep& R) {
 
 
 
+// Arrival slots for at least `cells` bags and up to `most`; none above
+// RANK_MAX_CELLS bags.  Every rebuild works without them, by segments or the
+// general sort, so a failure leaves none and is no error; a request as large is
+// not made again.
+void make_slots(kb_field* f, uint64_t cells, uint64_t most) {
+    f->slots_kept = false;
+    if (cells > RANK_MAX_CELLS) return;
+    most = std::min<uint64_t>(most, RANK_MAX_CELLS);
+    if (cells >= f->slots_refused) {
+        f->slots.release();
+        return;
+    }
+    if (f->slots.alloc((size_t)most * RANK_SLOTS) == cudaSuccess) return;
+    if (most > cells && f->slots.alloc((size_t)cells * RANK_SLOTS) == cudaSuccess) return;
+    f->slots_refused = cells;
+}
+
+// Give the arrival slots back: they are wanted less than what is allocated next.
+bool drop_slots(kb_field* f) {
+    if (f->slots.n == 0) return false;
+    f->slots.release();
+    f->slots_kept = false;
+    f->drop_graphs();  // captured over them
+    return true;
+}
+
 kb_status grow(kb_field* f, uint32_t need) {
     if (need <= f->cap) return KB_OK;
     if (f->virt) {
@@ -214,8 +240,12 @@ kb_status grow(kb_field* f, uint32_t need) {
     DevBuf<uint8_t> wdead;
     const size_t part = ((size_t)c + 3u) / 4u * 4u;  // 16-byte parts
     cudaError_t e;
-    if ((e = recs.alloc(3 * (size_t)c)) || (e = words.alloc(5 * part)) || (e = wdead.alloc(c)))
-        return cuda_fail(e, "growing object storage");
+    do {
+        e = recs.alloc(3 * (size_t)c);
+        if (!e) e = words.alloc(5 * part);
+        if (!e) e = wdead.alloc(c);
+    } while (e == cudaErrorMemoryAllocation && drop_slots(f));
+    if (e) return cuda_fail(e, "growing object storage");
     rst.view(recs.p, c);
     wst.view(recs.p + c, c);
     tst.view(recs.p + 2 * (size_t)c, c);
@@ -1121,7 +1151,6 @@ kb_status field_new(int device, const std::vector<Rep>& reps, bool is_batch, uin
     if (!e) e = f->start[0].alloc((size_t)nc + 1);
     if (!e) e = f->start[1].alloc((size_t)nc + 1);
     if (!e) e = f->hist.alloc(nc);
-    if (!e && nc <= RANK_MAX_CELLS) e = f->slots.alloc((size_t)nc * RANK_SLOTS);
     if (!e) e = f->scan_ctl.alloc(1);
     if (!e) e = f->aux_ctl.alloc(1);
     if (!e) e = f->tstate.alloc(nt);
@@ -1142,6 +1171,7 @@ kb_status field_new(int device, const std::vector<Rep>& reps, bool is_batch, uin
         delete f;
         return cuda_fail(e, "creating field");
     }
+    make_slots(f, nc, nc);
     if (kb_status st = build_rep_blocks(f)) {
         delete f;
         return st;
@@ -1164,13 +1194,16 @@ kb_status grow_cells(kb_field* f, uint64_t need) {
     if (need > 0xF0000000ull) return fail(KB_ERR_ARG, "bag matrix too large");
     const uint32_t nc = (uint32_t)std::min<uint64_t>(0xF0000000ull, std::max<uint64_t>(need, 2ull * f->cells_cap));
     const uint32_t nt = scan_state_words(nc);
-    DevBuf<uint32_t> s0, s1, hist, slots;
+    DevBuf<uint32_t> s0, s1, hist;
     DevBuf<unsigned long long> ts;
     cudaError_t e;
-    if ((e = s0.alloc((size_t)nc + 1)) || (e = s1.alloc((size_t)nc + 1)) || (e = hist.alloc(nc)) ||
-        (e = ts.alloc(nt)) ||
-        (nc <= RANK_MAX_CELLS && (e = slots.alloc((size_t)nc * RANK_SLOTS))))
-        return cuda_fail(e, "growing the bag arrays");
+    do {
+        e = s0.alloc((size_t)nc + 1);
+        if (!e) e = s1.alloc((size_t)nc + 1);
+        if (!e) e = hist.alloc(nc);
+        if (!e) e = ts.alloc(nt);
+    } while (e == cudaErrorMemoryAllocation && drop_slots(f));
+    if (e) return cuda_fail(e, "growing the bag arrays");
     KB_CUDA(cudaMemsetAsync(s0.p, 0, sizeof(uint32_t) * ((size_t)nc + 1), f->stream));
     KB_CUDA(cudaMemsetAsync(s1.p, 0, sizeof(uint32_t) * ((size_t)nc + 1), f->stream));
     KB_CUDA(cudaMemsetAsync(hist.p, 0, sizeof(uint32_t) * nc, f->stream));
@@ -1179,12 +1212,13 @@ kb_status grow_cells(kb_field* f, uint64_t need) {
     f->start[0].swap(s0);
     f->start[1].swap(s1);
     f->hist.swap(hist);
-    f->slots.swap(slots);
     f->tstate.swap(ts);
     f->cells_cap = nc;
     f->hist_counted = false;
     f->fused.ready = false;
     f->drop_graphs();
+    f->slots.release();
+    make_slots(f, nc, nc);
     return KB_OK;
 }
 
@@ -1212,9 +1246,8 @@ kb_status field_set_reps(kb_field* f, const std::vector<Rep>& reps) {
     // 690,000 boids in 31 requests; 32 requests 24.4 against 21.3 ms).
     // Doubled, so that a batch that grows request by request allocates a few
     // times only.
-    const size_t need = (size_t)total * RANK_SLOTS;
-    if (total <= RANK_MAX_CELLS && f->slots.n < need)
-        (void)f->slots.alloc(std::max(need, std::min<size_t>(2 * f->slots.n, (size_t)RANK_MAX_CELLS * RANK_SLOTS)));
+    if (f->slots.n < (size_t)total * RANK_SLOTS)
+        make_slots(f, total, std::max<uint64_t>(total, 2 * f->slots.n / RANK_SLOTS));
     return build_rep_blocks(f);
 }
 
@@ -1248,12 +1281,15 @@ kb_status kb_debug_allocation_counts(uint64_t* allocs, uint64_t* frees) try {
     return kb::exception_status();
 }
 
-kb_status kb_debug_fail_allocations(uint32_t count) try {
+kb_status kb_debug_fail_allocations_after(uint32_t skip, uint32_t count) try {
+    g_fail_skip.store((long long)skip, std::memory_order_relaxed);
     g_fail_allocs.store((long long)count, std::memory_order_relaxed);
     return KB_OK;
 } catch (...) {
     return kb::exception_status();
 }
+
+kb_status kb_debug_fail_allocations(uint32_t count) { return kb_debug_fail_allocations_after(0, count); }
 
 kb_status kb_field_create(const kb_field_desc* desc, kb_field** out) try {
     if (!desc || !out) return fail(KB_ERR_ARG, "null argument");

@@ -63,6 +63,7 @@ struct kb_field {
     // where that is above RANK_MAX_CELLS bags, of the bags a batch uses (too
     // short for the bag matrix, or empty: rebuilt by segments)
     DevBuf<uint32_t> slots;
+    uint64_t slots_refused = ~0ull;  // as many bags' slots did not fit in memory (make_slots)
     bool slots_kept = false;  // the last force pass left its arrivals in slots
     bool hist_counted = false;  // a force pass has counted arrivals into hist (no scan since)
     // Every replica's ids are distinct in the read buffer (checked on the

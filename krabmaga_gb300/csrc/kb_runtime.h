@@ -19,8 +19,9 @@ namespace kb {
 extern std::atomic<unsigned long long> g_dev_allocs, g_dev_frees;
 // Allocation-failure injection (kb_debug_fail_allocations): while positive,
 // each device allocation fails as if the device were out of memory, without
-// calling cudaMalloc, and takes one off the count.
-extern std::atomic<long long> g_fail_allocs;
+// calling cudaMalloc, and takes one off the count.  The first g_fail_skip
+// allocations are made as usual.
+extern std::atomic<long long> g_fail_allocs, g_fail_skip;
 
 template <typename T>
 struct DevBuf {
@@ -35,6 +36,7 @@ struct DevBuf {
         release();
         if (count == 0) return cudaSuccess;
         if (g_fail_allocs.load(std::memory_order_relaxed) > 0 &&
+            g_fail_skip.fetch_sub(1, std::memory_order_relaxed) <= 0 &&
             g_fail_allocs.fetch_sub(1, std::memory_order_relaxed) > 0)
             return cudaErrorMemoryAllocation;
         g_dev_allocs.fetch_add(1, std::memory_order_relaxed);
