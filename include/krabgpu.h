@@ -440,7 +440,8 @@ typedef struct kb_server kb_server;
 typedef struct {
     int32_t device;
     uint32_t max_slots;         /* requests running at once */
-    uint64_t hbm_budget_bytes;  /* device-state budget for running requests */
+    uint64_t hbm_budget_bytes;  /* device-state budget for running requests; what they leave of it
+                                   may hold a faster rebin's workspace (48 bytes per bag in use) */
     uint32_t quantum_steps;     /* longest epoch between admissions (0 = 100) */
     uint32_t max_request_boids; /* largest request (sizes the device pool) */
     uint32_t max_request_cells; /* largest request bag matrix */

@@ -199,14 +199,15 @@ bool fast_rebin_ok(const Rep& R) {
 
 
 // Arrival slots for at least `cells` bags and up to `most`; none above
-// RANK_MAX_CELLS bags.  Every rebuild works without them, by segments or the
-// general sort, so a failure leaves none and is no error; a request as large is
-// not made again.
+// RANK_MAX_CELLS bags or above slots_limit bytes.  Every rebuild works without
+// them, by segments or the general sort, so a failure leaves none and is no
+// error; a request as large is not made again.
 void make_slots(kb_field* f, uint64_t cells, uint64_t most) {
     f->slots_kept = false;
     if (cells > RANK_MAX_CELLS) return;
-    most = std::min<uint64_t>(most, RANK_MAX_CELLS);
-    if (cells >= f->slots_refused) {
+    const uint64_t limit = f->slots_limit / (RANK_SLOTS * sizeof(uint32_t));
+    most = std::min<uint64_t>(most, std::min<uint64_t>(limit, RANK_MAX_CELLS));
+    if (cells >= f->slots_refused || cells > limit) {
         f->slots.release();
         return;
     }
@@ -1125,7 +1126,7 @@ int32_t kb_device_count(void) {
 
 // Allocate a field over a replica table (cell_off/boid_off already set).
 kb_status field_new(int device, const std::vector<Rep>& reps, bool is_batch, uint32_t capacity,
-                    kb_field** out, uint32_t cells_cap) {
+                    kb_field** out, uint32_t cells_cap, uint64_t slots_limit) {
     *out = nullptr;
     int ndev = kb_device_count();
     if (ndev <= 0) return fail(KB_ERR_NO_DEVICE, "no CUDA device visible");
@@ -1143,6 +1144,7 @@ kb_status field_new(int device, const std::vector<Rep>& reps, bool is_batch, uin
     f->ncells_total = ncells;
     f->cells_cap = nc;
     f->is_batch = is_batch;
+    f->slots_limit = slots_limit;
     assign_segments(f->reps);
     f->rep = f->reps[0];
     cudaError_t e = cudaStreamCreateWithFlags(&f->stream, cudaStreamNonBlocking);
@@ -1240,13 +1242,13 @@ kb_status field_set_reps(kb_field* f, const std::vector<Rep>& reps) {
     f->drop_graphs();
     KB_CUDA(cudaMemcpyAsync(f->d_rep.p, f->reps.data(), sizeof(Rep) * reps.size(), cudaMemcpyHostToDevice, f->stream));
     KB_CUDA(cudaStreamSynchronize(f->stream));
-    // A field whose bag capacity is above RANK_MAX_CELLS (a server: 64 slots of
-    // 2^21 bags) gets the arrival slots of the bags it uses; when they do not
-    // fit in memory it rebins by segments (28 us a step against 14 to 20 at
-    // 690,000 boids in 31 requests; 32 requests 24.4 against 21.3 ms).
-    // Doubled, so that a batch that grows request by request allocates a few
-    // times only.
-    if (f->slots.n < (size_t)total * RANK_SLOTS)
+    // A server, and a field whose bag capacity is above RANK_MAX_CELLS, gets the
+    // arrival slots of the bags it uses; when they do not fit in memory, or in
+    // what the running requests leave of a server's budget, it rebins by
+    // segments (28 us a step against 14 to 20 at 690,000 boids in 31 requests;
+    // 32 requests 24.4 against 21.3 ms).  Doubled, so that a batch that grows
+    // request by request allocates a few times only.
+    if (f->slots.n < (size_t)total * RANK_SLOTS || f->slots.n * sizeof(uint32_t) > f->slots_limit)
         make_slots(f, total, std::max<uint64_t>(total, 2 * f->slots.n / RANK_SLOTS));
     return build_rep_blocks(f);
 }

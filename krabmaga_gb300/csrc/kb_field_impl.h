@@ -60,9 +60,10 @@ struct kb_field {
     // step temporaries
     DevBuf<uint32_t> hist, tid, tsrc, rkey, tkey;  // rkey, tkey: the tiled steps' only
     // arrival slots of the ranked rebin, RANK_SLOTS per bag of the capacity or,
-    // where that is above RANK_MAX_CELLS bags, of the bags a batch uses (too
-    // short for the bag matrix, or empty: rebuilt by segments)
+    // of a server and where that is above RANK_MAX_CELLS bags, of the bags a
+    // batch uses (too short for the bag matrix, or empty: rebuilt by segments)
     DevBuf<uint32_t> slots;
+    uint64_t slots_limit = ~0ull;  // bytes they may take (a server: what its requests leave of the budget)
     uint64_t slots_refused = ~0ull;  // as many bags' slots did not fit in memory (make_slots)
     bool slots_kept = false;  // the last force pass left its arrivals in slots
     bool hist_counted = false;  // a force pass has counted arrivals into hist (no scan since)
@@ -226,7 +227,8 @@ bool params_ok(const kb_flock_params* p, std::string* why);
 
 // Allocate a field over a replica table (cell_off / boid_off already set).
 kb_status field_new(int device, const std::vector<Rep>& reps, bool is_batch, uint32_t capacity,
-                    kb_field** out, uint32_t cells_cap = 0);
+                    kb_field** out, uint32_t cells_cap = 0,
+                    uint64_t slots_limit = ~0ull);
 // Object storage for at least `need` records / bag arrays for `need` bags.
 kb_status grow(kb_field* f, uint32_t need);
 kb_status grow_cells(kb_field* f, uint64_t need);

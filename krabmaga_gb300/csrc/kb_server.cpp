@@ -47,7 +47,9 @@ struct SrvReq {
 };
 
 uint64_t request_bytes(const Rep& R, uint32_t n) {
-    // read buffer + two write lists + sort scratch per boid; offsets per bag
+    // read buffer + two write lists + sort scratch per boid; offsets per bag.
+    // The arrival slots (48 B a bag in use) are not charged: they take what the
+    // running requests leave of the budget, or are left out.
     return (uint64_t)n * (16 + 4) * 6 + (uint64_t)R.ncells * 4 * 4;
 }
 
@@ -117,6 +119,10 @@ kb_status srv_repack(kb_server* S, std::vector<SrvReq*>& act) {
         if (e) return cuda_fail(e, "repack plan");
     }
     KB_CUDA(cudaMemcpyAsync(S->plan.p, plan.data(), sizeof(PackEntry) * plan.size(), cudaMemcpyHostToDevice, f->stream));
+    {
+        std::lock_guard<std::mutex> lk(S->mu);
+        f->slots_limit = S->desc.hbm_budget_bytes - std::min(S->used_bytes, S->desc.hbm_budget_bytes);
+    }
     // the old read buffer (rst) is the copy source; the write list the target
     if ((st = field_set_reps(f, reps))) return st;  // synchronises the stream (plan copied)
     KB_CUDA(launch_repack(S->plan.p, (int32_t)plan.size(), (uint32_t)boids, f->d_rep.p, f->rst.p, f->rid.p,
@@ -315,7 +321,7 @@ kb_status kb_server_create(const kb_server_desc* desc, kb_server** out) try {
     if (!make_rep_geometry(16.0f, 16.0f, 4.0f, 1, &R, &why)) return fail(KB_ERR_ARG, why);
     kb_field* f = nullptr;
     kb_status st = field_new(desc->device, std::vector<Rep>{R}, true, (uint32_t)cap, &f,
-                             (uint32_t)std::max<uint64_t>(cells, R.ncells));
+                             (uint32_t)std::max<uint64_t>(cells, R.ncells), 0);
     if (st) return st;
     kb_server* S = new kb_server();
     S->desc = *desc;

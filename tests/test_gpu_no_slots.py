@@ -107,3 +107,22 @@ def test_a_batch_that_grows_without_slots(gpu):
             assert same(b.get_replica(1), oracle_after(late.state, 6, 300.0, late.params))
         b.close()
     assert fewer >= 1
+
+
+@pytest.mark.parametrize("max_cells", [1 << 14, 1 << 24])
+def test_a_server_keeps_slots_within_its_budget(gpu, max_cells):
+    """A request that fills the budget runs by segments; with room, by ranks."""
+    n, side = 3000, 400.0
+    r = kg.Request(n, side, D, 40, kg.FlockParams(seed=5, arith=kg.KB_ARITH_FAST), 11)
+    cells = (int(np.ceil(np.float32(side) / np.float32(D))) + 1) ** 2
+    one = 120 * n + 16 * cells
+    out = []
+    for budget in (one + 47 * cells, one + 48 * cells):
+        with kg.Server(max_slots=8, quantum_steps=8, max_request_boids=n, max_request_cells=max_cells,
+                       hbm_budget_bytes=budget) as srv:
+            a = L.allocation_counts()[0]
+            t = srv.submit(r)
+            srv.wait_idle(60.0)
+            out.append((srv.result(t, n), L.allocation_counts()[0] - a))
+    assert same(out[0][0], out[1][0])
+    assert out[1][1] == out[0][1] + 1
