@@ -545,27 +545,33 @@ uint32_t* rank_slots(const kb_field* f) {
     return f->dense && f->reps.size() == 1 ? nullptr : field_slots(f);
 }
 
-// The general stable sort: write list -> read buffer (any list: counted here).
-kb_status general_rebuild(kb_field* f) {
+// The general stable sort: write list -> read buffer.  counted: the list is one
+// whole force pass, whose counts are in hist (and whose arrivals in slots, if it
+// kept them); any other list is counted here.
+kb_status general_rebuild(kb_field* f, bool counted) {
     cudaStream_t s = f->stream;
     const int nxt = 1 - f->cur;
-    // a force pass may have counted the list
-    if (f->hist_counted) KB_CUDA(cudaMemsetAsync(f->hist.p, 0, sizeof(uint32_t) * f->ncells_total, s));
+    const uint32_t* slots = counted ? (f->slots_kept ? f->slots.p : nullptr) : field_slots(f);
+    if (!counted) {
+        // a force pass may have counted the list before it was edited
+        if (f->hist_counted) KB_CUDA(cudaMemsetAsync(f->hist.p, 0, sizeof(uint32_t) * f->ncells_total, s));
+        KB_CUDA(launch_count_list(f->wkey.p, f->wdead.p, f->wn, f->hist.p, field_slots(f), f->ncells_total, f->tid.p, s));
+    }
     f->hist_counted = false;  // the scan below zeroes it
     f->slots_kept = false;
-    KB_CUDA(launch_count_list(f->wkey.p, f->wdead.p, f->wn, f->hist.p, field_slots(f), f->ncells_total, f->tid.p, s));
     KB_CUDA(launch_scan(f->hist.p, f->start[nxt].p, f->ncells_total, f->scan_ctl.p, f->tstate.p, f->err.p, true, s,
                         scan_wait(f)));
     PlaceArgs a{};
     a.key = f->wkey.p;
-    a.dead = f->wdead.p;
+    a.dead = counted ? nullptr : f->wdead.p;
     a.st = f->wst.p;
     a.ids = f->wid.p;
     a.n = f->wn;
-    a.arrival = f->tid.p;
+    a.arrival = counted ? nullptr : f->tid.p;
+    a.cursor = f->hist.p;
     a.start = f->start[nxt].p;
     a.ncells = f->ncells_total;
-    a.slots = field_slots(f);
+    a.slots = slots;
     a.order = f->tsrc.p;
     a.s_st = f->rst.p;
     a.s_ids = f->rid.p;
@@ -1088,12 +1094,12 @@ kb_status field_lazy_update(kb_field* f) {
     if (f->w_from_compute && !f->w_has_dead) {
         const bool stencil = all_fast_rebin_ok(f) && f->layout_is_positions;
         if (stencil || rank_any(f)) st = fast_rebuild(f, false, stencil);
-        else st = general_rebuild(f);
+        else st = general_rebuild(f, true);
         if (st) return st;
         f->rn = f->wn;
         f->layout_is_positions = true;
     } else {
-        st = general_rebuild(f);
+        st = general_rebuild(f, false);
         if (st) return st;
         if ((st = load_facts(f, f->wn))) return st;
     }
@@ -2281,7 +2287,7 @@ kb_status enqueue_steps(kb_field* f, const kb_flock_params* p, uint32_t nsteps, 
         f->wn = f->rn;
         f->kt_cur = t;
         const bool ranked = !fast && rank_any(f);
-        st = fast || ranked ? fast_rebuild(f, true, fast) : general_rebuild(f);
+        st = fast || ranked ? fast_rebuild(f, true, fast) : general_rebuild(f, true);
         f->kt_cur = -1;
         if (st) return st;
         if (t >= 0) KB_CUDA(cudaEventRecord(f->kt_pending[t].ev[3], f->stream));

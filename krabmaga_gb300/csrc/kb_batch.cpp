@@ -416,7 +416,7 @@ static kb_status batch_repack(kb_batch* b, std::vector<Rep> reps, const std::vec
     f->w_has_dead = false;
     f->virt = false;
     f->p_st.clear(); f->p_id.clear(); f->p_key.clear();
-    if ((st = general_rebuild(f))) return st;
+    if ((st = general_rebuild(f, false))) return st;
     f->wn = 0;
     if ((st = load_facts(f, (uint32_t)boids))) return st;
     f->rn = (uint32_t)boids;

@@ -238,7 +238,7 @@ kb_status upload_rep(kb_field* f);
 // Rebuild a virtual read buffer (after tiled steps).
 kb_status materialize(kb_field* f);
 // The general stable sort of the write list into the read buffer.
-kb_status general_rebuild(kb_field* f);
+kb_status general_rebuild(kb_field* f, bool counted);
 // Field::lazy_update (field_2d.rs:905-921).
 kb_status field_lazy_update(kb_field* f);
 // nsteps steps on the separate kernels (fast: the stencil-gather rebin).

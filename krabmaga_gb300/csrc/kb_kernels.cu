@@ -1368,7 +1368,9 @@ __global__ void k_canon(const uint32_t* __restrict__ start, uint32_t ncells,
 // bags of at most RANK_SLOTS arrivals at once (as k_rebin_rank); an entry of a
 // fuller bag (or of any shared bag, without slots) leaves its index at the
 // bag's offset plus its arrival number, and k_place_fuller puts each such bag
-// in list order, a warp per bag.  Bound by the scattered writes.  Scattering
+// in list order, a warp per bag.  A whole force pass has counted its list and
+// kept the slots already; only the entries of fuller bags then take an arrival
+// number, from the counts that the scan has zeroed.  Bound by the scattered writes.  Scattering
 // every record and then ordering each bag by one thread (quadratic in the bag)
 // took 52 us of a load of 1M uniform boids and 570 of 4M clustered ones; loads
 // with their steps and reads: 1M x 100 steps 4415 -> 4278 us, 4M clustered x 10
@@ -1393,10 +1395,12 @@ __global__ void __launch_bounds__(256) k_place_list(PlaceArgs a) {
     if (i >= a.n || (a.dead && a.dead[i])) return;
     const uint32_t key = a.key[i];
     const float4 rec = a.st[i];
-    const uint32_t id = a.ids[i], r = a.arrival[i];
-    const uint32_t s = a.start[key], c = a.start[key + 1] - s;
+    const uint32_t id = a.ids[i], r0 = a.arrival ? a.arrival[i] : 0u;
+    // (offsets of a scan whose wait ran out read as k_place_fuller reads them)
+    const uint32_t e = min(a.start[key + 1], a.n), s = min(a.start[key], e), c = e - s;
     uint32_t rank = 0;
     if (c > (a.slots ? RANK_SLOTS : 1u)) {
+        const uint32_t r = a.arrival ? r0 : atomicAdd(&a.cursor[key], 1u);
         if (s + r < a.n) a.order[s + r] = i;
         return;
     }
@@ -1428,7 +1432,9 @@ __global__ void __launch_bounds__(256) k_place_fuller(PlaceArgs a) {
         first = min(a.start[c], e);
         cnt = e - first;
     }
-    uint32_t todo = __ballot_sync(FULL_MASK, cnt > (a.slots ? RANK_SLOTS : 1u));
+    const bool fuller = cnt > (a.slots ? RANK_SLOTS : 1u);
+    if (fuller && !a.arrival) a.cursor[c] = 0u;  // zero again for the next count
+    uint32_t todo = __ballot_sync(FULL_MASK, fuller);
     // offsets of a scan whose wait ran out can claim bags of any length
     if (todo && (*((volatile uint32_t*)a.err) & ERR_SPIN_TIMEOUT)) return;
     while (todo) {

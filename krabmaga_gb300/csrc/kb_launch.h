@@ -238,7 +238,8 @@ cudaError_t launch_pack_states(const Rep& rep, const float4* st, uint32_t n, flo
 // The general rebuild: counts (hist zero before; arrival[i] = entry i's arrival
 // number, the bags' first RANK_SLOTS arrivals into slots unless nullptr), and
 // after the offsets scan every live entry to its place in list order.  order:
-// n words of scratch.
+// n words of scratch.  A list that a force pass counted has no arrival numbers
+// (nullptr): fuller bags take them from cursor, zero before and after.
 struct PlaceArgs {
     const uint32_t* key;
     const uint8_t* dead;
@@ -246,6 +247,7 @@ struct PlaceArgs {
     const uint32_t* ids;
     uint32_t n;
     const uint32_t* arrival;
+    uint32_t* cursor;
     const uint32_t* start;
     uint32_t ncells;
     const uint32_t* slots;

@@ -131,7 +131,7 @@ kb_status srv_repack(kb_server* S, std::vector<SrvReq*>& act) {
     f->w_from_compute = false;
     f->w_has_dead = false;
     f->virt = false;
-    if ((st = general_rebuild(f))) return st;
+    if ((st = general_rebuild(f, false))) return st;
     f->rn = (uint32_t)boids;
     set_ids_unique(f, true);  // every request's boids are ids 0..n-1
     f->wn = 0;
