@@ -107,11 +107,22 @@ struct ForceArgs {
 };
 // Up to how many boids the warp-per-boid kernel is the faster one: it gives a
 // boid 32 lanes, k_flock_force gives it one and waits for its columns in turn.
-// Measured (us per step, warp / thread per boid): 7 columns 8k 12.0 / 16.9, 20k
-// 18.2 / 18.0, 32k 24.7 / 18.4; 41 columns 1k 10.1 / 47, 20k 31 / 59; exact, 7
-// columns 8k 14.8 / 64.7, 41 columns 20k 45 / 764 (a corner rule per bag).
+// The general kernel's time hardly grows with the flock up to 64k boids and
+// grows with the columns, the warp-per-boid kernel's the other way round, so the
+// line lies by columns.  us per step, warp / thread per boid, density 0.025:
+//   relaxed, 5 columns  8k 10.8 / 13.2, 12k 12.5 / 13.3, 14k 13.7 / 13.7, 16k 15.1 / 14.1
+//            (strict 12.4 / 15.9, 15.2 / 16.1, 16.6 / 16.5, 18.2 / 16.8)
+//            7          8k 11.3 / 16.1, 16k 15.3 / 15.8, 32k 24.7 / 18.4
+//            21         16k 17.9 / 32.7, 32k 27.6 / 35.5
+//            41         1k 10.1 / 47, 20k 31 / 59
+//   exact,   5          33k 35 / 45, 40k 42 / 45, 49k 50 / 45, 262k 227 / 92 (strict 40k 48 / 48)
+//            7          66k 64 / 76, 98k 93 / 84, 262k 231 / 148 (strict 66k 74 / 81)
+//            9          131k 124 / 141 (strict 142 / 151)
+//            11         262k 243 / 310; 17: 275 / 590; 41: 131k 342 / 1098 (a corner rule per bag)
+// The same at densities 0.01 and 0.06.
 inline uint32_t wide_max(int32_t dd, int32_t qmode) {
-    return qmode != 0 ? 262144u : (2 * dd + 1 >= 16 ? 32768u : 16384u);
+    if (qmode != 0) return dd <= 2 ? 40000u : (dd == 3 ? 65536u : (dd == 4 ? 131072u : 262144u));
+    return dd <= 2 ? 12288u : (2 * dd + 1 >= 16 ? 32768u : 16384u);
 }
 constexpr int FORCE_THREADS = 256;  // the force kernel's block (one replica per block)
 // Block sizes of the force pass over packed replicas (one replica per block).
