@@ -390,13 +390,18 @@ void occ_poll(kb_field* f) {
 
 // Whole steps in one cluster (kb_small.cu): a plain field small enough for
 // shared memory, on the default step path.  Wide rings leave it where the
-// warp-per-boid kernel takes them (1,000 boids, 7 columns: 8.2 us a step against
-// 12.3, exact 8.5 against 52).
+// warp-per-boid kernel takes them (us per step, cluster / warp per boid: 1,000
+// boids, 5 columns 7.0 / 7.4, strict 8.0 / 7.7, at density 0.06 9.0 / 7.6, exact
+// 31 / 8.1; 7 columns 12.3 / 8.2, exact 52 / 8.5) and, crowded, where the walk by
+// runs and the segments beat it (dense relaxed, 5 and 7 columns: 1,000 boids 53
+// / 58, 2,000 45 / 49 and 59 / 46, 4,000 50 / 45 and 80 / 58; exact 1,000 134 /
+// 165, 2,000 107 / 129, 4,000 134 / 131).
 bool small_eligible(const kb_field* f) {
     const Rep& R = f->reps[0];
+    const bool stays = R.dd <= 1 || !R.nowrap || !f->ids_unique ||
+                       (f->dense && (R.qmode != KB_QUERY_RELAX || f->rn < SMALL_DENSE_WIDE));
     return !f->is_batch && f->reps.size() == 1 && f->fused_mode == 0 && !f->virt && f->rn > 0 &&
-           f->rn <= SMALL_MAX_BOIDS && R.ncells <= SMALL_MAX_CELLS && R.cell_off == 0 &&
-           !(R.dd > 1 && R.nowrap && f->ids_unique);
+           f->rn <= SMALL_MAX_BOIDS && R.ncells <= SMALL_MAX_CELLS && R.cell_off == 0 && stays;
 }
 
 // Bag rows and segment count of the segment rebin.

@@ -59,3 +59,23 @@ def test_both_sides_of_the_wide_rule_match_oracle(gpu, n, d, kind, over):
     f.flock_step(p, 0, 2)
     assert same(f.get_state(), after(side, d, birds, p, 2))
     f.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,kind,path", [(600, RELAX, kg.KB_PATH_SMALL), (600, EXACT, kg.KB_PATH_SMALL),
+                                         (1999, RELAX, kg.KB_PATH_SMALL), (2000, RELAX, kg.KB_PATH_DENSE),
+                                         (2000, EXACT, kg.KB_PATH_SMALL), (4096, EXACT, kg.KB_PATH_SMALL)])
+def test_dense_wide_rings_of_small_fields(gpu, n, kind, path):
+    # crowded: the warp-per-boid kernel, for which wide rings leave the cluster, is not taken
+    side, d = float(np.float32(np.sqrt(n / 1.0))), 4.0
+    side = max(side, 32.0)
+    birds = kg.gen_clustered(n, side, side, 1, 6.0, 0.5, 3)
+    p = kg.FlockParams(seed=2, arith=kg.KB_ARITH_STRICT, query_mode=kind, neighbor_radius=10.0)
+    f = kg.Field2D(side, side, d, True)
+    f.set_locations(*birds)
+    f.lazy_update()
+    f.flock_step(p, 0, 2)
+    f.flock_step(p, 2, 2)
+    assert f.dense_active() and f.step_path() == path
+    assert same(f.get_state(), after(side, d, birds, p, 4))
+    f.close()
