@@ -1110,10 +1110,15 @@ __global__ void __launch_bounds__(32 * REBIN_SEG_WARPS, MULTI ? KB_REBIN_MINB_MU
 // Fuller bags: the warp takes its distinct keys in turn; for each it reads the
 // bag's source lines, and every lane of that key counts the arrivals before its
 // own entry.  A chain of dependent loads bounds it, so the lanes look their own
-// bags' replicas and columns up together before the first key, and an interior
+// bags' replicas and columns up together before the first key, an interior
 // bag's three columns are read as one list, 128 entries in flight (bounds and
 // columns in turn per key, 32 entries at a time: 32 requests 21.5 ms against
-// 20.6, 64 condensing replicas 58.3 against 57.4 ms).  Every lane of the warp calls it with its
+// 20.6), and a bag at the seam or the edge has the bounds of all its lines
+// loaded at once, a run per lane (line by line, up to 64 pairs of dependent
+// loads, such bags held the whole step up as soon as a few were fuller: 64 x
+// 4,096 boids at density 0.25 103 us a step, now 48, 64-bag segments 45; 16 x
+// 65,536 with four crowded ones 162, 130, 167; 64 condensing replicas 96, 89,
+// 101).  Every lane of the warp calls it with its
 // entry i (over: the entry's bag is a fuller one).  Out of line and after the
 // others are written, so that it costs them no registers.
 // The source lines hold every arrival unless one has moved past them.  Each
@@ -1123,6 +1128,7 @@ template <bool MULTI>
 __device__ __noinline__ void place_by_lines(const RebinArgs& a, bool over, uint32_t i) {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t key = 0, first = 0, rank = 0;
+    int rep = 0;
     // an interior bag's source columns, entries [s, e) each, ascending
     uint32_t s0 = 0, e0 = 0, s1 = 0, e1 = 0, s2 = 0, e2 = 0;
     bool inner = false, seen = a.any_move != 0;
@@ -1130,7 +1136,8 @@ __device__ __noinline__ void place_by_lines(const RebinArgs& a, bool over, uint3
         key = __ldcg(a.key + i);
         first = __ldg(a.start_next + key);
         if (!a.any_move) {
-            const Rep& R = MULTI ? a.reps[rep_of_cell(a.reps, a.nrep, key)] : a.rep0;
+            if (MULTI) rep = rep_of_cell(a.reps, a.nrep, key);
+            const Rep& R = MULTI ? a.reps[rep] : a.rep0;
             const uint32_t local = key - R.cell_off, dh = (uint32_t)R.dh;
             const uint32_t Xu = div_dh(local, R);
             const int X = (int)Xu, Y = (int)(local - Xu * dh);
@@ -1179,41 +1186,76 @@ __device__ __noinline__ void place_by_lines(const RebinArgs& a, bool over, uint3
             }
             continue;
         }
-        const Rep& R = MULTI ? a.reps[rep_of_cell(a.reps, a.nrep, k)] : a.rep0;
-        const uint32_t local = k - R.cell_off;
-        const uint32_t Xu = div_dh(local, R);
-        const int X = (int)Xu, Y = (int)(local - Xu * (uint32_t)R.dh);
-        auto count = [&](uint32_t s, uint32_t end) {
-            seen |= mine && i - s < end - s;
-            const uint32_t e = min(end, last);
+        if (a.any_move) {
 #pragma unroll 2
-            for (uint32_t p = s; p < e; p += 32u) {
-                const bool hit = p + lane < e && __ldg(a.key + p + lane) == k;
+            for (uint32_t p = 0; p < last; p += 32u) {
+                const bool hit = p + lane < last && __ldg(a.key + p + lane) == k;
                 const uint32_t m = __ballot_sync(FULL_MASK, hit);
                 // entries p .. i-1 of this batch
                 const uint32_t d = i > p ? i - p : 0u;
                 rank += mine ? __popc(d >= 32u ? m : m & ((1u << d) - 1u)) : 0;
             }
-        };
-        if (a.any_move) {
-            count(0u, a.n);
-        } else {
-            int lastx = -1;
+            continue;
+        }
+        // a bag at the seam or the field's edge: its source lines are up to
+        // three runs of rows in up to six columns (src_line's, ascending), a
+        // run per lane, and together one list, 64 entries in flight
+        const Rep& R = MULTI ? a.reps[__shfl_sync(FULL_MASK, rep, leader)] : a.rep0;
+        const uint32_t local = k - R.cell_off;
+        const uint32_t Xu = div_dh(local, R);
+        const int X = (int)Xu, Y = (int)(local - Xu * (uint32_t)R.dh);
+        const int sx = src_line((int)(lane >> 2), X, R.max_x, R.seam), part = (int)(lane & 3u);
+        int ra = 0, rb = -1;
+        if (part == 0 && Y >= R.seam) rb = 0;  // bags from the seam on take row 0
+        if (part == 1) ra = max(0, Y - 1), rb = min(R.max_y, Y + 1);
+        if (part == 2 && Y == 0) ra = R.seam, rb = min(R.seam + SRC_LINES - 5, R.max_y);  // row 0 takes the seam's rows
+        uint32_t s = 0, len = 0;
+        if (sx >= 0 && sx <= R.max_x && ra <= rb) {
+            const uint32_t* c = a.start_cur + R.cell_off + (uint32_t)sx * (uint32_t)R.dh;
+            const uint32_t e = min(min(__ldg(c + rb + 1), a.n), last + 1u);
+            s = min(__ldg(c + ra), e);
+            len = e - s;
+        }
+        uint32_t incl = len;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL_MASK, incl, d);
+            if (lane >= (uint32_t)d) incl += y;
+        }
+        const uint32_t T = __shfl_sync(FULL_MASK, incl, 31);
+        s -= incl - len;  // entry f of the list is s + f, of the run that holds it
 #pragma unroll 1
-            for (int kx = 0; kx < SRC_LINES; ++kx) {
-                const int sx = src_line(kx, X, R.max_x, R.seam);
-                if (sx < 0 || sx > R.max_x || sx <= lastx) continue;
-                lastx = sx;
-                const uint32_t colbase = R.cell_off + (uint32_t)sx * (uint32_t)R.dh;
-                int lasty = -1;
-#pragma unroll 1
-                for (int ky = 0; ky < SRC_LINES; ++ky) {
-                    const int sy = src_line(ky, Y, R.max_y, R.seam);
-                    if (sy < 0 || sy > R.max_y || sy <= lasty) continue;
-                    lasty = sy;
-                    const uint32_t e = min(__ldg(a.start_cur + colbase + sy + 1), a.n);
-                    count(min(__ldg(a.start_cur + colbase + sy), e), e);
+        for (uint32_t p = 0; p < T; p += 64u) {
+            uint32_t at[2];
+            bool hit[2];
+#pragma unroll
+            for (uint32_t u = 0; u < 2; ++u) {
+                const uint32_t f = p + 32u * u + lane;
+                // the first run whose inclusive count exceeds f
+                uint32_t q = 0;
+#pragma unroll
+                for (uint32_t d = 16; d > 0; d >>= 1) {
+                    const uint32_t y = __shfl_sync(FULL_MASK, incl, q + d - 1u);
+                    if (y <= f) q += d;
                 }
+                const uint32_t base = __shfl_sync(FULL_MASK, s, q);
+                at[u] = f < T ? base + f : 0xFFFFFFFFu;
+                hit[u] = f < T && __ldg(a.key + at[u]) == k;
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < 2; ++u) {
+                const uint32_t m = __ballot_sync(FULL_MASK, hit[u]);
+                // the list ascends: how many of these 32 stand before entry i
+                uint32_t d = 0;
+#pragma unroll
+                for (uint32_t h = 16; h > 0; h >>= 1) {
+                    const uint32_t y = __shfl_sync(FULL_MASK, at[u], d + h - 1u);
+                    if (y < i) d += h;
+                }
+                const uint32_t y = __shfl_sync(FULL_MASK, at[u], d);
+                seen |= mine && y == i;
+                if (y < i) ++d;
+                rank += mine ? __popc(d >= 32u ? m : m & ((1u << d) - 1u)) : 0;
             }
         }
     }
