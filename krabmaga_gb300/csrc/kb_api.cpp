@@ -354,19 +354,24 @@ unsigned long long* pinned_page(kb_field* f) {
     return f->occ_host;
 }
 
+// The device words of what loads and running steps measure, made at the first load
+// so that no step allocates.
+kb_status facts_words(kb_field* f) {
+    cudaError_t e = cudaSuccess;
+    if (f->facts.n < FACT_WORDS) e = f->facts.alloc(FACT_WORDS);
+    if (!e && !f->occ_ev) e = cudaEventCreateWithFlags(&f->occ_ev, cudaEventDisableTiming);
+    return e ? cuda_fail(e, "load facts") : KB_OK;
+}
+
 // Enqueue a measurement of the read buffer into the pinned word (no wait).
 kb_status occ_enqueue(kb_field* f) {
     if (f->reps.size() != 1 || f->virt) return KB_OK;
     if (!pinned_page(f)) return KB_OK;  // no measurement: the flag stays as it is
-    if (!f->occ_ev) {
-        cudaError_t e = f->occ_dev.alloc(1);
-        if (!e) e = cudaEventCreateWithFlags(&f->occ_ev, cudaEventDisableTiming);
-        if (e) return cuda_fail(e, "occupancy measurement");
-    }
-    KB_CUDA(cudaMemsetAsync(f->occ_dev.p, 0, sizeof(unsigned long long), f->stream));
-    KB_CUDA(launch_occupancy_sq(f->start[f->cur].p, f->ncells_total, f->occ_dev.p, f->stream));
-    KB_CUDA(cudaMemcpyAsync(f->occ_host + PIN_OCC, f->occ_dev.p, sizeof(unsigned long long),
-                            cudaMemcpyDeviceToHost, f->stream));
+    if (kb_status st = facts_words(f)) return st;
+    unsigned long long* word = f->facts.p + FACT_OCC;
+    KB_CUDA(cudaMemsetAsync(word, 0, sizeof(unsigned long long), f->stream));
+    KB_CUDA(launch_occupancy_sq(f->start[f->cur].p, f->ncells_total, word, f->stream));
+    KB_CUDA(cudaMemcpyAsync(f->occ_host + PIN_OCC, word, sizeof(unsigned long long), cudaMemcpyDeviceToHost, f->stream));
     KB_CUDA(cudaEventRecord(f->occ_ev, f->stream));
     f->occ_pending = true;
     f->occ_n = f->rn;
@@ -1068,8 +1073,8 @@ kb_status load_facts(kb_field* f, uint32_t most) {
     const size_t words = (size_t)most / 32u + 1u;
     cudaError_t e = cudaSuccess;
     if (f->id_bits.n < words) e = f->id_bits.alloc(words);
-    if (!e && f->facts.n < 3) e = f->facts.alloc(3);
     if (e) return cuda_fail(e, "load facts");
+    if (kb_status st = facts_words(f)) return st;
     unsigned long long local[3];
     unsigned long long* r = pinned_page(f) ? f->occ_host + PIN_FACTS : local;
     KB_CUDA(cudaMemsetAsync(f->id_bits.p, 0, sizeof(uint32_t) * words, f->stream));

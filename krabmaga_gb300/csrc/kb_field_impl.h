@@ -22,6 +22,8 @@ using namespace kb;
 // Words of a field's pinned page: the occupancy measurement of running steps, the
 // three results of a load, a word read back.
 enum { PIN_OCC = 0, PIN_FACTS = 1, PIN_WORD = 4, PIN_WORDS = 8 };
+// Device words: the three results of a load, the occupancy measurement of running steps.
+enum { FACT_OCC = 3, FACT_WORDS = 4 };
 
 struct kb_field {
     int device = 0;
@@ -72,7 +74,7 @@ struct kb_field {
     bool ids_unique = false;
     DevBuf<unsigned long long> dup_tab;  // hash table, only for ids past the replica's boid count
     DevBuf<uint32_t> id_bits;            // a bit per record: the ids below it that were seen
-    DevBuf<unsigned long long> facts;    // launch_load_facts' results
+    DevBuf<unsigned long long> facts;    // launch_load_facts' results, and FACT_OCC
     // Several replicas: block tables of the force and segment-rebin kernels
     // ({replica, first boid} / {replica, first segment}), no block spanning
     // two replicas; rebuilt with the replica table.
@@ -166,7 +168,6 @@ struct kb_field {
     // (read back without blocking).  Both paths give the same bits.
     int32_t dense_mode = KB_DENSE_AUTO;
     bool dense = false;
-    DevBuf<unsigned long long> occ_dev;
     unsigned long long* occ_host = nullptr;  // pinned: PIN_* words
     cudaEvent_t occ_ev = nullptr;
     bool occ_pending = false;
