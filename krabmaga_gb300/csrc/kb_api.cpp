@@ -62,19 +62,16 @@ kb_status cuda_fail(cudaError_t e, const char* what) {
 
 // Host copy of discretize + bag index (field_2d.rs:328-339, 840-841) for
 // argument checks on API writes; the same IEEE f32 operations as the device.
-int64_t host_bag_index(const Rep& R, float x, float y) {
+// *inside (if given): whether the position's own column and row are lines of the
+// matrix.  The bag index of another one can still lie inside it: a bag of some
+// other column.
+int64_t host_bag_index(const Rep& R, float x, float y, bool* inside) {
     int32_t cx = as_i32(std::floor(x / R.d));
     int32_t cy = as_i32(std::floor(y / R.d));
     int32_t idx = (int32_t)((uint32_t)cx * (uint32_t)R.dh + (uint32_t)cy);
+    if (inside) *inside = (uint32_t)cx <= (uint32_t)R.max_x && (uint32_t)cy <= (uint32_t)R.max_y;
     if (idx < 0 || (uint32_t)idx >= R.ncells) return -1;
     return idx;
-}
-
-// Whether a position's own column and row are lines of the matrix.  The bag
-// index of another one can still lie inside it: a bag of some other column.
-bool host_inside(const Rep& R, float x, float y) {
-    const int32_t cx = as_i32(std::floor(x / R.d)), cy = as_i32(std::floor(y / R.d));
-    return cx >= 0 && cx <= R.max_x && cy >= 0 && cy <= R.max_y;
 }
 
 bool make_rep_geometry(float w, float h, float d, int toroidal, Rep* R, std::string* why,
@@ -1362,7 +1359,8 @@ kb_status kb_field_set_object_location(kb_field* f, uint32_t id, const float pos
     f->p_st.push_back(make_float4(pos[0], pos[1], last_d[0], last_d[1]));
     f->p_id.push_back(id);
     f->p_key.push_back((uint32_t)idx);
-    if (host_bag_index(f->rep, pos[0], pos[1]) != idx || !host_inside(f->rep, pos[0], pos[1])) f->p_loc_differs = true;
+    bool inside = false;
+    if (host_bag_index(f->rep, pos[0], pos[1], &inside) != idx || !inside) f->p_loc_differs = true;
     if (!f->density_check) f->nagents += 1;
     f->w_from_compute = false;
     return KB_OK;

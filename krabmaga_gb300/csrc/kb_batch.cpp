@@ -104,13 +104,15 @@ kb_status kb_batch_set_replica(kb_batch* b, uint32_t r, size_t n, const uint32_t
     if (n != f->reps[r].nboids) return fail(KB_ERR_ARG, "boid count differs from the replica's nboids");
     const Rep& R = f->reps[r];
     const size_t old = f->p_id.size();
+    bool all_inside = true;
     for (size_t i = 0; i < n; ++i) {
         if (!(std::isfinite(xy[2 * i]) && std::isfinite(xy[2 * i + 1]) && std::isfinite(dxy[2 * i]) &&
               std::isfinite(dxy[2 * i + 1]))) {
             f->p_st.resize(old); f->p_id.resize(old); f->p_key.resize(old);
             return fail(KB_ERR_ARG, "non-finite position or heading");
         }
-        const int64_t idx = host_bag_index(R, xy[2 * i], xy[2 * i + 1]);
+        bool inside = false;
+        const int64_t idx = host_bag_index(R, xy[2 * i], xy[2 * i + 1], &inside);
         if (idx < 0) {
             f->p_st.resize(old); f->p_id.resize(old); f->p_key.resize(old);
             return fail(KB_ERR_RANGE, "location outside the replica's bag matrix");
@@ -118,8 +120,9 @@ kb_status kb_batch_set_replica(kb_batch* b, uint32_t r, size_t n, const uint32_t
         f->p_st.push_back(make_float4(xy[2 * i], xy[2 * i + 1], dxy[2 * i], dxy[2 * i + 1]));
         f->p_id.push_back(ids[i]);
         f->p_key.push_back(R.cell_off + (uint32_t)idx);
-        if (!host_inside(R, xy[2 * i], xy[2 * i + 1])) f->p_loc_differs = true;
+        all_inside &= inside;
     }
+    if (!all_inside) f->p_loc_differs = true;
     b->have[r] = 1;
     return KB_OK;
 } catch (...) {

@@ -217,8 +217,7 @@ struct DeviceGuard {
 namespace kb {
 extern thread_local std::string g_last_error;  // kb_last_error()'s message for this thread
 // Host copy of discretize + bag index (field_2d.rs:328-339): -1 outside the matrix.
-int64_t host_bag_index(const Rep& R, float x, float y);
-bool host_inside(const Rep& R, float x, float y);
+int64_t host_bag_index(const Rep& R, float x, float y, bool* inside = nullptr);
 // Field2D::new geometry (field_2d.rs:304-322) into R; false with *why on bad input.
 bool make_rep_geometry(float w, float h, float d, int toroidal, Rep* R, std::string* why,
                        int cell_wrap = KB_CELL_WRAP_CLAMP);
