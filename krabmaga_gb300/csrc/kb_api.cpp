@@ -342,6 +342,21 @@ void set_dense(kb_field* f, bool d) {
     f->dense = d;
 }
 
+// Packed replicas: whether most boids stand in bags fuller than the arrival slots.
+// By ranks each such bag's arrivals are counted by the warps that hold them, by
+// segments the bag is gathered in one pass.  us per step, ranks / 64-bag segments
+// (share of the boids in such bags): 16 replicas of 65,536, uniform, 111 / 129
+// (0.16), 145 / 144 (0.75), 179 / 176 (0.99); 64 of 16,384 clustered 114 / 120
+// (0.29), 136 / 141 (0.44), 177 / 177 (0.62); small batches, where the longest
+// warp counts, 64 of 1,024 46 / 39 (0.64), 4 of 8,192 65 / 48 (0.78).
+bool crowded_from(unsigned long long full, uint32_t n) { return n > 0 && 5ull * full >= 3ull * n; }
+
+// A finished measurement of the read buffer: how dense it is.
+void set_occupancy(kb_field* f, unsigned long long v, uint32_t n) {
+    if (f->reps.size() == 1) set_dense(f, dense_from(v, n));
+    else f->crowded = crowded_from(v, n);
+}
+
 // The field's page of pinned words, made on first use (nullptr: none to be had).
 unsigned long long* pinned_page(kb_field* f) {
     if (!f->occ_host && cudaMallocHost(&f->occ_host, sizeof(unsigned long long) * PIN_WORDS) != cudaSuccess) {
@@ -362,15 +377,16 @@ kb_status facts_words(kb_field* f) {
 
 // Enqueue a measurement of the read buffer into the pinned word (no wait).
 kb_status occ_enqueue(kb_field* f) {
-    if (f->reps.size() != 1 || f->virt) return KB_OK;
+    if (f->virt) return KB_OK;
     if (!pinned_page(f)) return KB_OK;  // no measurement: the flag stays as it is
     if (kb_status st = facts_words(f)) return st;
     unsigned long long* word = f->facts.p + FACT_OCC;
     KB_CUDA(cudaMemsetAsync(word, 0, sizeof(unsigned long long), f->stream));
-    KB_CUDA(launch_occupancy_sq(f->start[f->cur].p, f->ncells_total, word, f->stream));
+    KB_CUDA(launch_occupancy_sq(f->start[f->cur].p, f->ncells_total, f->reps.size() == 1 ? 0u : RANK_SLOTS, word, f->stream));
     KB_CUDA(cudaMemcpyAsync(f->occ_host + PIN_OCC, word, sizeof(unsigned long long), cudaMemcpyDeviceToHost, f->stream));
     KB_CUDA(cudaEventRecord(f->occ_ev, f->stream));
     f->occ_pending = true;
+    f->occ_packed = f->reps.size() > 1;
     f->occ_n = f->rn;
     f->steps_since_occ = 0;
     return KB_OK;
@@ -387,7 +403,18 @@ void occ_poll(kb_field* f) {
         return;
     }
     f->occ_pending = false;
-    set_dense(f, dense_from(f->occ_host[PIN_OCC], f->occ_n));
+    // (a batch's replicas may have changed since: a measurement of the other kind says nothing)
+    if (f->occ_packed == (f->reps.size() > 1)) set_occupancy(f, f->occ_host[PIN_OCC], f->occ_n);
+}
+
+// Take or start the measurement of packed replicas that are about to step.
+kb_status occ_refresh(kb_field* f, uint64_t steps) {
+    if (f->reps.size() == 1) return KB_OK;
+    occ_poll(f);
+    kb_status st = KB_OK;
+    if (!f->occ_pending && f->steps_since_occ >= DENSE_REFRESH) st = occ_enqueue(f);
+    f->steps_since_occ += steps;
+    return st;
 }
 
 // Whole steps in one cluster (kb_small.cu): a plain field small enough for
@@ -545,11 +572,12 @@ uint32_t* field_slots(const kb_field* f) {
 }
 
 // The arrival slots a force pass keeps for the ranked rebin; nullptr for dense
-// flocks, which rebin by segments: most of their boids share a bag with more
-// than RANK_SLOTS others, and every key of a warp would walk its source lines
-// (4M clustered boids: rebin 238 us by ranks, 160 us by 8-bag segments).
+// flocks and crowded batches, which rebin by segments: most of their boids share
+// a bag with more than RANK_SLOTS others, and every key of a warp would walk its
+// source lines (4M clustered boids: rebin 238 us by ranks, 160 us by 8-bag
+// segments; crowded_from for packed replicas).
 uint32_t* rank_slots(const kb_field* f) {
-    return f->dense && f->reps.size() == 1 ? nullptr : field_slots(f);
+    return (f->reps.size() == 1 ? f->dense : f->crowded) ? nullptr : field_slots(f);
 }
 
 // The general stable sort: write list -> read buffer.  counted: the list is one
@@ -1062,11 +1090,10 @@ kb_status check_unique_hashed(kb_field* f) {
 }
 
 // After a general rebuild of `most` records at most: how many are stored, how
-// dense a plain field is, and whether ids are distinct within each replica, in
+// dense they are, and whether ids are distinct within each replica, in
 // one launch and one read (ids below their replica's boid count, the usual
 // ones, are marked in a bitmap; others are compared by hashing after it).
 kb_status load_facts(kb_field* f, uint32_t most) {
-    const bool plain = f->reps.size() == 1;
     const size_t words = (size_t)most / 32u + 1u;
     cudaError_t e = cudaSuccess;
     if (f->id_bits.n < words) e = f->id_bits.alloc(words);
@@ -1077,16 +1104,14 @@ kb_status load_facts(kb_field* f, uint32_t most) {
     KB_CUDA(cudaMemsetAsync(f->id_bits.p, 0, sizeof(uint32_t) * words, f->stream));
     KB_CUDA(cudaMemsetAsync(f->facts.p, 0, sizeof(unsigned long long) * 3, f->stream));
     KB_CUDA(launch_load_facts(f->d_rep.p, nrep(f), most, f->rid.p, f->start[f->cur].p,
-                              plain ? f->ncells_total : 0u, f->start[f->cur].p + f->ncells_total, most,
+                              f->ncells_total, f->start[f->cur].p + f->ncells_total, most,
                               f->id_bits.p, f->facts.p, f->stream));
     KB_CUDA(cudaMemcpyAsync(r, f->facts.p, sizeof(unsigned long long) * 3, cudaMemcpyDeviceToHost, f->stream));
     KB_CUDA(cudaStreamSynchronize(f->stream));
     f->rn = (uint32_t)r[2];
-    if (plain) {
-        f->occ_pending = false;
-        f->steps_since_occ = 0;
-        set_dense(f, dense_from(r[0], f->rn));
-    }
+    f->occ_pending = false;
+    f->steps_since_occ = 0;
+    set_occupancy(f, r[0], f->rn);
     if ((r[1] & 3ull) == 2ull) return check_unique_hashed(f);
     set_ids_unique(f, r[1] == 0ull);
     return KB_OK;

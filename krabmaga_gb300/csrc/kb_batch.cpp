@@ -171,7 +171,10 @@ kb_status kb_batch_step(kb_batch* b, uint64_t first_step, uint32_t nsteps, uint3
         if ((st = materialize(f))) return st;
         if ((st = grow(f, f->rn))) return st;
         const bool fast = all_fast_rebin_ok(f) && f->layout_is_positions;
-        if (graph_launches <= 1 || !fast) return enqueue_steps(f, p, nsteps, fast);
+        if (graph_launches <= 1 || !fast) {
+            if ((st = occ_refresh(f, nsteps))) return st;
+            return enqueue_steps(f, p, nsteps, fast);
+        }
         // separate-kernel steps replayed from CUDA graphs of up to graph_launches
         // steps (the kernels read the step number from device memory, so one
         // capture serves every step range)
@@ -182,6 +185,7 @@ kb_status kb_batch_step(kb_batch* b, uint64_t first_step, uint32_t nsteps, uint3
         uint32_t done = 0;
         while (done < nsteps) {
             const uint32_t k = std::min(graph_launches, nsteps - done);
+            if ((st = occ_refresh(f, k))) return st;
             if (k < 4) {
                 if ((st = enqueue_steps(f, p, k, fast))) return st;
                 done += k;
@@ -189,7 +193,7 @@ kb_status kb_batch_step(kb_batch* b, uint64_t first_step, uint32_t nsteps, uint3
             }
             const uint64_t sig = ((uint64_t)f->force_block << 48) ^ ((uint64_t)f->nblk_force << 24) ^
                                  (uint64_t)f->nblk_seg ^ ((uint64_t)f->rn << 8) ^
-                                 (f->ids_unique ? (1ull << 63) : 0ull);
+                                 (f->ids_unique ? (1ull << 63) : 0ull) ^ (f->crowded ? (1ull << 62) : 0ull);
             kb_batch::GKey key{k, 0u, f->cur, 0, 0, sig};
             auto it = b->graphs.find(key);
             const int cur0 = f->cur;

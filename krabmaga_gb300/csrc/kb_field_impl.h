@@ -168,9 +168,11 @@ struct kb_field {
     // (read back without blocking).  Both paths give the same bits.
     int32_t dense_mode = KB_DENSE_AUTO;
     bool dense = false;
+    bool crowded = false;  // packed replicas: rebuilt by segments (crowded_from)
     unsigned long long* occ_host = nullptr;  // pinned: PIN_* words
     cudaEvent_t occ_ev = nullptr;
     bool occ_pending = false;
+    bool occ_packed = false;  // of several replicas
     uint32_t occ_n = 0;  // boids when the pending measurement was taken
     uint64_t steps_since_occ = 0;
 
@@ -263,7 +265,9 @@ kb_status autotune_force_block(kb_field* f, uint64_t first_step, uint32_t steps,
                                const int32_t* cand, int32_t ncand, int32_t* best_out,
                                float* best_ms_out, kb_status (*run)(void*, uint64_t, uint32_t),
                                void* ctx);
-// After a general rebuild: the stored count, a plain field's density and whether
+// Before `steps` steps of packed replicas on the separate kernels: how crowded they are.
+kb_status occ_refresh(kb_field* f, uint64_t steps);
+// After a general rebuild: the stored count, the field's density and whether
 // every replica's ids are distinct (one read back) / set the last.
 kb_status load_facts(kb_field* f, uint32_t most);
 void set_ids_unique(kb_field* f, bool u);

@@ -1343,13 +1343,17 @@ __global__ void __launch_bounds__(RANK_THREADS, MULTI ? 6 : 8) k_rebin_rank(Rebi
 
 // Sum of squared bag occupancies of a read buffer (its offsets), a measure
 // of how long the candidate lists are: about 9 * sum / N per boid.
-__global__ void k_occupancy_sq(const uint32_t* __restrict__ start, uint32_t ncells,
+// fuller > 0: the objects in bags of more than `fuller` instead.
+__device__ __forceinline__ unsigned long long occupancy_term(unsigned long long o, uint32_t fuller) {
+    return fuller ? (o > fuller ? o : 0ull) : o * o;
+}
+__global__ void k_occupancy_sq(const uint32_t* __restrict__ start, uint32_t ncells, uint32_t fuller,
                                unsigned long long* out) {
     __shared__ unsigned long long s_part[8];
     unsigned long long acc = 0;
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += gridDim.x * blockDim.x) {
         const unsigned long long o = (unsigned long long)(start[c + 1] - start[c]);
-        acc += o * o;
+        acc += occupancy_term(o, fuller);
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) acc += __shfl_down_sync(FULL_MASK, acc, d);
@@ -1501,8 +1505,8 @@ __global__ void __launch_bounds__(256) k_place_fuller(PlaceArgs a) {
 
 // What a load of the read buffer has to know, in one launch and one read back:
 // (an 8 B hash slot per id, cleared each time, took 34 us at 1M ids):
-// res[0] the sum of squared bag occupancies (bags over a plain field; 0 for
-// ncells 0), res[1] bit 0: an id below its replica's boid count repeats (its
+// res[0] the sum of squared bag occupancies (packed replicas: the objects in bags
+// of more than RANK_SLOTS; 0 for ncells 0), res[1] bit 0: an id below its replica's boid count repeats (its
 // bit in `bits`), bit 1: some id is not below it (the caller compares by
 // hashing), res[2] the objects stored.  res and bits are cleared by the caller.
 __global__ void __launch_bounds__(256)
@@ -1533,7 +1537,7 @@ __global__ void __launch_bounds__(256)
     unsigned long long acc = 0;
     for (uint32_t c = g; c < ncells; c += step) {
         const unsigned long long o = (unsigned long long)(start[c + 1] - start[c]);
-        acc += o * o;
+        acc += occupancy_term(o, nrep > 1 ? RANK_SLOTS : 0u);
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) acc += __shfl_down_sync(FULL_MASK, acc, d);
@@ -2133,12 +2137,12 @@ cudaError_t launch_rebin(const RebinArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_occupancy_sq(const uint32_t* start, uint32_t ncells, unsigned long long* out,
+cudaError_t launch_occupancy_sq(const uint32_t* start, uint32_t ncells, uint32_t fuller, unsigned long long* out,
                                 cudaStream_t s) {
     if (ncells == 0) return cudaSuccess;
     const unsigned g0 = grid_for(ncells, 256);
     const unsigned g = g0 < 608u ? g0 : 608u;  // grid-stride: four blocks per SM of 152
-    k_occupancy_sq<<<g, 256, 0, s>>>(start, ncells, out);
+    k_occupancy_sq<<<g, 256, 0, s>>>(start, ncells, fuller, out);
     return cudaGetLastError();
 }
 

@@ -222,8 +222,9 @@ inline uint32_t rep_segments(const Rep& R, int rows = 0) {
     return (uint32_t)R.dw * (((uint32_t)R.dh + (uint32_t)rows - 1) / (uint32_t)rows);
 }
 cudaError_t launch_rebin(const RebinArgs& a, cudaStream_t s);
-// *out += sum over bags of (start[c+1] - start[c])^2 (the caller zeroes *out).
-cudaError_t launch_occupancy_sq(const uint32_t* start, uint32_t ncells, unsigned long long* out,
+// *out += sum over bags of (start[c+1] - start[c])^2, or with fuller > 0 the
+// objects in bags of more than `fuller` (the caller zeroes *out).
+cudaError_t launch_occupancy_sq(const uint32_t* start, uint32_t ncells, uint32_t fuller, unsigned long long* out,
                                 cudaStream_t s);
 // Whether any (replica, id) pair repeats in the read buffer (n boids, nrep
 // replicas by boid_off): an open-addressing table of cap (a power of two,
@@ -271,7 +272,8 @@ struct PlaceArgs {
 cudaError_t launch_count_list(const uint32_t* key, const uint8_t* dead, uint32_t n, uint32_t* hist,
                               uint32_t* slots, uint32_t ncells, uint32_t* arrival, cudaStream_t s);
 cudaError_t launch_place_list(const PlaceArgs& a, cudaStream_t s);
-// res[0..2] = {sum of squared bag occupancies over ncells bags, id flags (1 a
+// res[0..2] = {sum of squared bag occupancies over ncells bags (several replicas:
+// the objects in bags of more than RANK_SLOTS), id flags (1 a
 // repeat among the ids below their replica's boid count, 2 an id that is not
 // below it), objects stored}; bits: one bit per record (cap of them), cleared
 // with res by the caller.  nboids0: the boid count of a single replica.

@@ -196,7 +196,8 @@ bool srv_epoch(kb_server* S, std::vector<SrvReq*>& act, bool& changed) {
         if (fused_eligible(f, &S->common)) {
             st = tiled_steps(f, &S->common, K);
         } else {
-            if (!(st = materialize(f))) st = enqueue_steps(f, &S->common, K, all_fast_rebin_ok(f));
+            if (!(st = materialize(f)) && !(st = occ_refresh(f, K)))
+                st = enqueue_steps(f, &S->common, K, all_fast_rebin_ok(f));
         }
         S->launches++;
     }
