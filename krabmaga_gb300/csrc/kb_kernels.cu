@@ -176,10 +176,8 @@ __device__ __forceinline__ void gather_candidates(const ForceArgs& a, const Rep&
                 columns_flat3<STRICT, DENSE>(a, R, mi, Mi, mj, Mj, me, my_id, acc, my_slot);
             else columns_runs_5(a, R, mi, Mi, mj, Mj, me, my_id, acc);
         } else {
-            // counted: a line number may be the greatest i32
-            const uint32_t ni = (uint32_t)Mi - (uint32_t)mi, nj = (uint32_t)Mj - (uint32_t)mj;
-            for (uint32_t u = 0; u <= ni; ++u) {
-                const int bx = t_transform((int)((uint32_t)mi + u), R.max_x);
+            for (int ci = mi; ci <= Mi; ++ci) {
+                const int bx = t_transform(ci, R.max_x);
                 const uint32_t colbase = R.cell_off + (uint32_t)bx * (uint32_t)R.dh;
                 if (QMODE == 0 && clamped) {
                     const uint32_t e = min(__ldg(a.start + colbase + Mj + 1), a.n);
@@ -187,8 +185,8 @@ __device__ __forceinline__ void gather_candidates(const ForceArgs& a, const Rep&
                                    my_id, acc);
                     continue;
                 }
-                for (uint32_t v = 0; v <= nj; ++v) {
-                    const int by = t_transform((int)((uint32_t)mj + v), R.max_y);
+                for (int cj = mj; cj <= Mj; ++cj) {
+                    const int by = t_transform(cj, R.max_y);
                     const uint32_t c = colbase + (uint32_t)by;
                     const uint32_t e = min(__ldg(a.start + c + 1), a.n);
                     const uint32_t s = min(__ldg(a.start + c), e);
@@ -1674,12 +1672,10 @@ __global__ void k_query(QueryArgs a) {
                query_ring<KIND>(a, p, mi, Mi, mj, Mj, off, fill, &cnt, &dig)) {
         // done
     } else {
-        // counted: a line number may be the greatest i32
-        const uint32_t ni = (uint32_t)Mi - (uint32_t)mi, nj = (uint32_t)Mj - (uint32_t)mj;
-        for (uint32_t u = 0; u <= ni; ++u) {
-            const int bx = t_transform((int)((uint32_t)mi + u), R.max_x);
-            for (uint32_t v = 0; v <= nj; ++v) {
-                const int by = t_transform((int)((uint32_t)mj + v), R.max_y);
+        for (int ci = mi; ci <= Mi; ++ci) {
+            const int bx = t_transform(ci, R.max_x);
+            for (int cj = mj; cj <= Mj; ++cj) {
+                const int by = t_transform(cj, R.max_y);
                 const uint32_t c = R.cell_off + (uint32_t)bx * (uint32_t)R.dh + (uint32_t)by;
                 const uint32_t s = a.start[c], e = a.start[c + 1];
                 if (s == e) continue;

@@ -48,7 +48,10 @@ int main() {
                     if (!cell_range(R, x, y, dd, &mi, &Mi, &mj, &Mj)) continue;
                     ++some;
                     // a walk may rely on it: lines of the matrix, none out of order
-                    if (mi > Mi || mj > Mj) ++bad;
+                    if (mi > Mi || mj > Mj || Mi == INT_MAX || Mj == INT_MAX) ++bad;
+                    // (a line moved to end the walk is the same one)
+                    else if (wrap && dd == 0 && (t_transform(mi, 100) != t_transform(disc(x, R), 100) ||
+                                                 t_transform(mj, 100) != t_transform(disc(y, R), 100))) ++bad;
                     else if (!wrap && (mi < 0 || Mi > 99 || mj < 0 || Mj > 99)) ++bad;
                 }
     std::printf("%%d %%d\n", bad, some > 0);
