@@ -1501,7 +1501,7 @@ __global__ void __launch_bounds__(256) k_place_fuller(PlaceArgs a) {
     }
 }
 
-// What a load of the read buffer has to know, in one launch and one read back:
+// What a load of the read buffer has to know, in one launch and one read back
 // (an 8 B hash slot per id, cleared each time, took 34 us at 1M ids):
 // res[0] the sum of squared bag occupancies (packed replicas: the objects in bags
 // of more than RANK_SLOTS; 0 for ncells 0), res[1] bit 0: an id below its replica's boid count repeats (its
@@ -1529,7 +1529,12 @@ __global__ void __launch_bounds__(256)
             flags |= 2u;
         }
     }
-    if (flags) atomicOr(res + 1, (unsigned long long)flags);
+    // one atomic per warp, and none for what is known already: with ids past the
+    // count, or repeated, every thread would come (loads of 200,000 such ids 295
+    // and 206 us, now 174 and 147)
+    flags = __reduce_or_sync(FULL_MASK, flags);
+    if ((threadIdx.x & 31u) == 0u && (flags & ~(uint32_t)*((volatile unsigned long long*)(res + 1))))
+        atomicOr(res + 1, (unsigned long long)flags);
     if (g == 0) res[2] = *total;
     if (ncells == 0) return;
     unsigned long long acc = 0;
