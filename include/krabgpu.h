@@ -229,8 +229,9 @@ kb_status kb_flock_step(kb_field* f, const kb_flock_params* p, uint64_t first_st
  * kernels (a plain field replays runs of 4 steps or more from CUDA graphs),
  * except that a plain field of at most 4096 boids and 4096 bags runs whole
  * steps in one 8-block thread-block cluster (shared memory, up to 1000 steps
- * per launch; not a call of one step with kernel timing on, nor rings wider
- * than one bag where the warp-per-boid kernel takes them);
+ * per launch; a call of one step only up to 1,200 boids and with kernel timing
+ * off, and rings wider than one bag only where neither the warp-per-boid
+ * kernel nor, from 2,000 crowded boids on, the dense walk is the faster);
  * 3 the separate kernels whatever the field's size;
  * for eligible fields (toroidal, square, jump < discretization) 2 the tiled
  * step as two launches per step (stage + rebin + force per tile, then the

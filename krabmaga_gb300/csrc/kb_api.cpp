@@ -2360,11 +2360,13 @@ static kb_status flock_step_impl(kb_field* f, const kb_flock_params* p, uint64_t
     }
     if (done < nsteps && fused_eligible(f, p)) return tiled_steps(f, p, nsteps - done);
     if (f->virt && (st = materialize(f))) return st;
-    if (small_eligible(f) && (nsteps - done >= 2 || !f->ktime)) {
+    if (small_eligible(f) && (nsteps - done >= 2 || (!f->ktime && f->rn <= SMALL_SINGLE_MAX))) {
         // a small field: whole steps in one cluster, up to 1000 per launch.  A
-        // single step too (a frame of 1,000 boids, step and state read: 47 us,
-        // 50 to 54 with the separate kernels' four launches), unless its kernels
-        // are being timed.
+        // single step too, unless its kernels are being timed: one launch
+        // instead of three, until the cluster's load and write-back cost more (a
+        // step waited for, cluster / separate kernels: 300 boids 25.3 / 26.9 us,
+        // 1,000 26.5 / 27.3, 1,500 27.1 / 26.7, 4,096 31.5 / 27.5; strict 27.3 /
+        // 28.5, 27.9 / 28.3, 32.8 / 29.3 from 1,000 on).
         while (done < nsteps) {
             const uint32_t k = std::min<uint32_t>(1000u, nsteps - done);
             SmallArgs a{};

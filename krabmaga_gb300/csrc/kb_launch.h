@@ -142,6 +142,7 @@ constexpr uint32_t SMALL_CTAS = 8;  // a portable cluster size
 // separate kernels; the bound is the shared memory.
 constexpr uint32_t SMALL_MAX_BOIDS = 4096;
 constexpr uint32_t SMALL_MAX_CELLS = 4096;
+constexpr uint32_t SMALL_SINGLE_MAX = 1200;  // boids up to which a single step takes the cluster
 constexpr uint32_t SMALL_DENSE_WIDE = 2000;  // from here on crowded wide rings of relaxed queries leave it
 struct SmallArgs {
     Rep rep;

@@ -79,3 +79,22 @@ def test_dense_wide_rings_of_small_fields(gpu, n, kind, path):
     assert f.dense_active() and f.step_path() == path
     assert same(f.get_state(), after(side, d, birds, p, 4))
     f.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", [RELAX, EXACT])
+@pytest.mark.parametrize("n", [1200, 1201, 4096])
+def test_single_steps_and_runs_of_small_fields_mix(gpu, n, kind):
+    # one step at a time on either side of the cluster's limit, runs between them
+    side, d = float(np.float32(np.sqrt(n / 0.025))), float(np.float32(10.0) / np.float32(1.5))
+    birds = kg.gen_uniform(n, side, side, 4, 1.0)
+    p = kg.FlockParams(seed=6, arith=kg.KB_ARITH_STRICT, query_mode=kind)
+    f = kg.Field2D(side, side, d, True)
+    f.set_locations(*birds)
+    f.lazy_update()
+    done = 0
+    for k in (1, 1, 3, 1, 5, 1):
+        f.flock_step(p, done, k)
+        done += k
+    assert same(f.get_state(), after(side, d, birds, p, done))
+    f.close()
