@@ -2142,7 +2142,7 @@ cudaError_t launch_occupancy_sq(const uint32_t* start, uint32_t ncells, uint32_t
                                 cudaStream_t s) {
     if (ncells == 0) return cudaSuccess;
     const unsigned g0 = grid_for(ncells, 256);
-    const unsigned g = g0 < 608u ? g0 : 608u;  // grid-stride: four blocks per SM of 152
+    const unsigned g = g0 < 4u * GB300_SMS ? g0 : 4u * GB300_SMS;  // grid-stride: four blocks per SM
     k_occupancy_sq<<<g, 256, 0, s>>>(start, ncells, fuller, out);
     return cudaGetLastError();
 }
@@ -2166,7 +2166,7 @@ cudaError_t launch_load_facts(const Rep* reps, int32_t nrep, uint32_t nboids0, c
                               uint32_t* bits, unsigned long long* res, cudaStream_t s) {
     const uint64_t most = cap > ncells ? cap : ncells;
     const unsigned g0 = grid_for(most > 0 ? most : 1, 256);
-    const unsigned g = g0 < 1216u ? g0 : 1216u;  // grid-stride: eight blocks per SM of 152
+    const unsigned g = g0 < 8u * GB300_SMS ? g0 : 8u * GB300_SMS;  // grid-stride: eight blocks per SM
     k_load_facts<<<g, 256, 0, s>>>(reps, nrep, nboids0, ids, start, ncells, total, cap, bits, res);
     return cudaGetLastError();
 }

@@ -18,6 +18,7 @@ struct ScanCtl {
     uint32_t epoch;
     uint32_t _pad;
 };
+constexpr unsigned GB300_SMS = 152;
 constexpr uint32_t SCAN_TILE = 4096;  // items per CTA (256 threads x 16)
 inline uint32_t scan_tiles(uint32_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE; }
 constexpr uint32_t SCAN_CLUSTER = 8;  // blocks of the one-launch cluster scan
@@ -97,8 +98,8 @@ struct ForceArgs {
     // several replicas: threads per block of the block table (FORCE_BLOCKS_*;
     // 0: FORCE_THREADS), the launch shape the batch autotuner picks
     uint32_t block_threads;
-    // every replica is a torus with the clamped range, no pair
-    // straddles the seam, the ring is at most one bag wide, ids are distinct
+    // every replica is a torus with the clamped range, no pair straddles the
+    // seam (Rep::nowrap, and every object in its own position's bag), the ring is at most one bag wide, ids are distinct
     // and n <= 2^26 (byte offsets of three runs in 32 bits): the ring kernels
     int32_t ring;
     // the same with a wider ring, one replica of at most wide_max boids: the

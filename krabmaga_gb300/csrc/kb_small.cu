@@ -18,7 +18,8 @@
 //      order), plus those of earlier warps of its chunk (one byte per warp and
 //      bag), plus its rank among its warp's equal keys (__match_any_sync): the
 //      reference's insertion order inside a bag.  Each record goes to the blocks
-//      whose next chunk can see its column (to all where queries wrap);
+//      whose next chunk can see its column (to all where queries wrap, or birds
+//      stand beyond the height);
 //   -- cluster barrier --
 // and every block writes its chunk of the final read buffer back.  No bound on
 // how far a boid moves is needed.
@@ -224,7 +225,6 @@ __host__ __device__ inline SmallLayout small_layout(uint32_t n, uint32_t ncells,
 constexpr uint32_t SMALL_OUTSIDE = 0xFFFFu;  // a key outside the matrix (its boid goes to bag 0)
 constexpr uint32_t SMALL_NONE = 0xFFFEu;     // no boid
 
-// T: threads per block, at least twice the chunk.
 // Shared memory of the cluster's blocks by 32-bit addresses.
 __device__ __forceinline__ uint32_t remote_address(const void* local, uint32_t rank) {
     uint32_t r;
@@ -240,6 +240,7 @@ __device__ __forceinline__ void store_remote(uint32_t at, uint32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at), "r"(v) : "memory");
 }
 
+// T: threads per block, at least twice the chunk.
 template <bool STRICT, int QMODE, int T>
 __global__ void __launch_bounds__(T, 1) k_small_steps(SmallArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
