@@ -137,6 +137,12 @@ __device__ __forceinline__ void columns_flat3(const ForceArgs& a, const Rep& R, 
             const float4 o = __ldg(a.st + p);
             if (oid != my_id) acc.template add<true>(R, me.x, me.y, o);
         }
+    } else if (my_slot != 0xFFFFFFFFu) {  // wrapped pairs (a field wider than high)
+        for (uint32_t f = 0; f < T; ++f) {
+            const uint32_t p = f < P1 ? s[0] + f : (f < P2 ? f + d1 : f + d2);
+            const float4 o = __ldg(a.st + p);
+            if (p != my_slot) acc.template add<false>(R, me.x, me.y, o);
+        }
     } else {
         for (uint32_t f = 0; f < T; ++f) {
             const uint32_t p = f < P1 ? s[0] + f : (f < P2 ? f + d1 : f + d2);
