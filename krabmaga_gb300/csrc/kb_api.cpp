@@ -378,8 +378,10 @@ kb_status facts_words(kb_field* f) {
 // Enqueue a measurement of the read buffer into the pinned word (no wait).
 kb_status occ_enqueue(kb_field* f) {
     if (f->virt) return KB_OK;
-    if (!pinned_page(f)) return KB_OK;  // no measurement: the flag stays as it is
-    if (kb_status st = facts_words(f)) return st;
+    if (!pinned_page(f) || facts_words(f)) {  // no measurement: the flag stays as it is
+        f->steps_since_occ = 0;
+        return KB_OK;
+    }
     unsigned long long* word = f->facts.p + FACT_OCC;
     KB_CUDA(cudaMemsetAsync(word, 0, sizeof(unsigned long long), f->stream));
     KB_CUDA(launch_occupancy_sq(f->start[f->cur].p, f->ncells_total, f->reps.size() == 1 ? 0u : RANK_SLOTS, word, f->stream));

@@ -6,6 +6,7 @@ import pytest
 
 import krabmaga_gb300 as kg
 import oracle
+from krabmaga_gb300 import _lib as L
 
 pytestmark = pytest.mark.gpu
 D = float(np.float32(10.0) / np.float32(1.5))
@@ -71,3 +72,28 @@ def test_crowded_requests(gpu):
             got, want = srv.result(t, r.nboids), f.get_state()
             assert np.array_equal(got[0], want[0]) and np.array_equal(got[1].view(np.uint32), want[1].view(np.uint32))
             f.close()
+
+
+def test_a_server_that_cannot_measure_goes_on(gpu):
+    """No memory for the measurement's words: the requests run all the same."""
+    def ask(n, side, steps):
+        return kg.Request(n, side, D, steps, kg.FlockParams(seed=n, arith=kg.KB_ARITH_FAST), n)
+
+    with kg.Server(max_slots=4, quantum_steps=8, max_request_boids=4000, max_request_cells=1 << 14) as srv:
+        # a larger batch first, for too few steps to be measured: all tables that the
+        # one below needs are there (one request alone, so that both join it)
+        srv.submit(ask(4000, 600.0, 16))
+        srv.submit(ask(3999, 600.0, 40))
+        srv.submit(ask(3998, 600.0, 40))
+        srv.wait_idle(60.0)
+        reqs = [ask(2000, 200.0, 160), ask(1500, 180.0, 200)]
+        L.fail_allocations(1)
+        try:
+            tickets = [srv.submit(r) for r in reqs]
+            srv.wait_idle(60.0)
+        finally:
+            L.fail_allocations(0)
+        for t, r in zip(tickets, reqs):
+            assert srv.poll(t)[0] == 2
+            ids, st = srv.result(t, r.nboids)
+            assert np.array_equal(np.sort(ids), np.arange(r.nboids)) and np.isfinite(st).all()
